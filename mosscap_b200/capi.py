@@ -195,6 +195,8 @@ def load() -> ctypes.CDLL:
     lib.mc_adjoint_set_slab_hook.restype = i32
     lib.mc_debug_reverse_reciprocal.argtypes = [vp, vp, i64, vp]
     lib.mc_debug_reverse_reciprocal.restype = i32
+    lib.mc_debug_exact_ops.argtypes = [i32, vp, vp, vp, i64, vp]
+    lib.mc_debug_exact_ops.restype = i32
     if lib.mc_abi_version() != 1:
         raise RuntimeError("unexpected ABI version")
     _LIB = lib

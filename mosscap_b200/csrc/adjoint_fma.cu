@@ -475,6 +475,7 @@ StageParams fwd_params(const mc_adjoint* a) {
     p.plane = a->plane;
     p.dx = a->grid.dx;
     p.gamma = a->scheme.gamma;
+    p.gas = mc::fast_gas(p.gamma);
     p.blk = a->blk;
     for (int f = 0; f < 6; ++f) {
         p.bc.kind[f] = f < 4 ? MC_BC_PERIODIC : MC_BC_USERFN;

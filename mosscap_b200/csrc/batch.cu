@@ -466,6 +466,7 @@ mc_status mc_batch_create(const mc_batch_problem* problems, int32_t n, const mc_
         p.plane = (long long)g.xc * g.yc;
         p.dx = g.dx;
         p.gamma = s.gamma;
+        p.gas = mc::fast_gas(s.gamma);
         p.dt_dev = &b->d_blocks[i].dt;
         p.blk = &b->d_blocks[i];
         for (int f = 0; f < 6; ++f) {

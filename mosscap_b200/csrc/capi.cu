@@ -122,6 +122,7 @@ StageParams base_params(const mc_ctx* c) {
     p.plane = c->plane;
     p.dx = c->grid.dx;
     p.gamma = c->scheme.gamma;
+    p.gas = mc::fast_gas(c->scheme.gamma);
     p.blk = c->blk;
     p.gravity = c->gravity;
     for (int a = 0; a < 3; ++a) {
@@ -1238,6 +1239,16 @@ mc_status mc_stage_time(mc_ctx* c, int32_t kind, double* total_ms, int64_t* laun
     }
     *total_ms = sum;
     *launches = n;
+    return MC_OK;
+}
+
+mc_status mc_debug_exact_ops(int32_t op, const double* a, const double* b, double* out, int64_t n, void* stream) {
+    if (!a || !out || n < 0 || op < 0 || op > 2 || (op == 0 && !b)) {
+        return fail(MC_ERR_INVALID_ARGUMENT, "null argument, negative count or unknown op");
+    }
+    if (n > 0) {
+        MC_CUDA(mc::launch_exact_ops(op, a, b, out, n, (cudaStream_t)stream), "exact ops");
+    }
     return MC_OK;
 }
 

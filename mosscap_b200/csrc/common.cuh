@@ -5,6 +5,7 @@
 
 #include <cstdint>
 
+#include "exact_fp64.cuh"
 #include "physics.cuh"
 
 namespace mc {
@@ -55,6 +56,7 @@ struct StageParams {
     int nvar, ntracer;
     long long plane;                  // xc * yc * zc
     double dx, gamma;
+    FastGas gas;                      // fast_gas(gamma)
     double dt;                        // used when dt_dev is null
     const double* dt_dev;             // device dt (the device-driven loop)
     int combo;

@@ -199,6 +199,7 @@ mc_status mc_time_step_noalloc(const mc_grid* grid, const mc_scheme* scheme, dou
         p.plane = (long long)g.xc * g.yc * g.zc;
         p.dx = g.dx;
         p.gamma = s.gamma;
+        p.gas = mc::fast_gas(s.gamma);
         p.dt = dt;
         p.dt_dev = nullptr;
         p.combo = plan.combo[k];

@@ -104,6 +104,12 @@ __device__ __forceinline__ long long qidx(const StageParams& p, int v, int k, in
 template <int NDIM, class T>
 __device__ __forceinline__ double cfl_bound_of(const StageParams& p, const double* q, unsigned* flags) {
     constexpr int nh = 2 + NDIM;
+    if constexpr (sizeof(T) == 8) {
+        double w[nh];
+        if (p.gas.ok && in_range_pos(p.dx) && fast_prim<NDIM>(p.gas.gm1, q, w)) {
+            return fast_cfl_dt<NDIM>(p.gamma, p.dx, w);  // in range: no flag to raise
+        }
+    }
     bool fin = true;
 #pragma unroll
     for (int v = 0; v < nh; ++v) {
@@ -281,10 +287,15 @@ __device__ __forceinline__ double write_cell(const StageParams& p, int i, int j,
 // |m|^2 / (2 rho), so that the cancellation E - e_kin of high-Mach and
 // near-vacuum cells stays an FP64 operation -- one FP64 division per cell
 // instead of 2 + (NDIM > 1) + (NDIM > 2).
+// Returns whether the cell is in range for the FP64 sweep (exact_fp64.cuh).
 template <int NDIM, class T>
-__device__ __forceinline__ void prim_for_sweep(double gamma, const double* q, double* w) {
+__device__ __forceinline__ bool prim_for_sweep(double gamma, const FastGas& gas, const double* q, double* w) {
     if constexpr (sizeof(T) == 8) {
-        prim_from_cons<NDIM>(gamma, q, w);
+        const bool ok = fast_prim<NDIM>(gas.gm1, q, w);
+        if (!ok) {
+            prim_from_cons<NDIM>(gamma, q, w);
+        }
+        return ok;
     } else {
         const double inv = 1.0 / q[0];
         double m2 = q[1] * q[1];
@@ -299,14 +310,16 @@ __device__ __forceinline__ void prim_for_sweep(double gamma, const double* q, do
             w[3] = q[3] * inv;
         }
         w[1 + NDIM] = (gamma - 1.0) * (q[1 + NDIM] - 0.5 * m2 * inv);
+        return true;
     }
 }
 
 // Load one cell's conserved variables from q_in and store its primitives
 // (tracers divided by rho, source/Hydro.cpp:27-33) into shared memory.
+// Clears in_range unless the cell is in range for the FP64 sweep.
 template <int NDIM, class T>
 __device__ __forceinline__ unsigned load_prim(const StageParams& p, int k, int j, int i, bool inb, T* w_smem,
-                                              int var_stride) {
+                                              int var_stride, bool& in_range) {
     constexpr int nh = 2 + NDIM;
     double q[nh], w[nh];
     const long long vs = (long long)p.zc * p.yc * p.xc;  // variable stride of the state
@@ -325,7 +338,8 @@ __device__ __forceinline__ unsigned load_prim(const StageParams& p, int k, int j
         }
         q[nh - 1] = 1.0;
     }
-    prim_for_sweep<NDIM, T>(p.gamma, q, w);
+    const bool ok = prim_for_sweep<NDIM, T>(p.gamma, p.gas, q, w);
+    in_range = in_range && ok;
 #pragma unroll
     for (int v = 0; v < nh; ++v) {
         w_smem[v * var_stride] = T(w[v]);
@@ -334,11 +348,15 @@ __device__ __forceinline__ unsigned load_prim(const StageParams& p, int k, int j
         const double inv_rho = 1.0 / q[0];
         for (int t = 0; t < p.ntracer; ++t) {
             const double qt = inb ? p.q_in[id0 + (nh + t) * vs] : 0.0;
-            w_smem[(nh + t) * var_stride] = T(qt * inv_rho);
+            const T s = T(qt * inv_rho);
+            w_smem[(nh + t) * var_stride] = s;
+            if constexpr (sizeof(T) == 8) {
+                in_range = in_range && in_range_any(s);
+            }
         }
     }
-    if (!inb) {
-        return 0u;
+    if (!inb || (sizeof(T) == 8 && ok)) {
+        return 0u;  // in range: no flag to raise
     }
     bool fin = true;
 #pragma unroll
@@ -352,7 +370,7 @@ __device__ __forceinline__ unsigned load_prim(const StageParams& p, int k, int j
 // TMA-staged tile (variable stride stg_vs doubles); no tracers.
 template <int NDIM, class T>
 __device__ __forceinline__ unsigned staged_prim(const StageParams& p, const double* src, int stg_vs, bool inb,
-                                                T* w_smem, int var_stride) {
+                                                T* w_smem, int var_stride, bool& in_range) {
     constexpr int nh = 2 + NDIM;
     double q[nh], w[nh];
     if (inb) {
@@ -369,13 +387,14 @@ __device__ __forceinline__ unsigned staged_prim(const StageParams& p, const doub
         }
         q[nh - 1] = 1.0;
     }
-    prim_for_sweep<NDIM, T>(p.gamma, q, w);
+    const bool ok = prim_for_sweep<NDIM, T>(p.gamma, p.gas, q, w);
+    in_range = in_range && ok;
 #pragma unroll
     for (int v = 0; v < nh; ++v) {
         w_smem[v * var_stride] = T(w[v]);
     }
-    if (!inb) {
-        return 0u;
+    if (!inb || (sizeof(T) == 8 && ok)) {
+        return 0u;  // in range: no flag to raise
     }
     bool fin = true;
 #pragma unroll
@@ -482,6 +501,131 @@ __device__ __forceinline__ void face_sweep(const T* centre, int stride, int vstr
     }
 }
 
+// face_sweep on double in a call of its own: d into out[0..nh), the tracers'
+// d_tr after it. The FP64 sweep's form for values out of range.
+template <int NDIM, int REC, int LIM, int RS>
+__device__ __noinline__ void face_sweep_any(const double* centre, int stride, int vstride, int ntracer, double gamma,
+                                            double gfac, int axis, double* out) {
+    constexpr int nh = 2 + NDIM;
+    double d[nh], d_tr[kMaxVars];
+    face_sweep<NDIM, REC, LIM, RS, double>(centre, stride, vstride, ntracer, gamma, gfac, axis, d, d_tr);
+#pragma unroll
+    for (int v = 0; v < nh; ++v) {
+        out[v] = d[v];
+    }
+    for (int t = 0; t < ntracer; ++t) {
+        out[nh + t] = d_tr[t];
+    }
+}
+
+// face_sweep for a stencil in range, with the branch-free physics of
+// exact_fp64.cuh (the same bits). False on a lane whose face states the
+// reconstruction left out of range; d holds no result then.
+template <int NDIM, int REC, int LIM, int RS>
+__device__ __forceinline__ bool fast_face_sweep(const double* centre, int stride, int vstride, int ntracer,
+                                                double gamma, const FastGas& gas, int axis, double* d, double* d_tr) {
+    constexpr int nh = 2 + NDIM;
+    constexpr int S = stencil_half<REC>();
+    constexpr int G = recon_group<NDIM, REC>();
+    double wl[nh], wr[nh];
+    if constexpr (G < nh) {
+        // rolled as in face_sweep
+#pragma unroll
+        for (int v = 0; v < nh; ++v) {
+            wl[v] = 0.0;
+            wr[v] = 0.0;
+        }
+#pragma unroll 1
+        for (int v0 = 0; v0 < nh; v0 += G) {
+            double a[G], b[G];
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                double s[5];
+#pragma unroll
+                for (int o = -S; o <= S; ++o) {
+                    s[2 + o] = centre[(v0 + g) * vstride + o * stride];
+                }
+                fast_reconstruct<REC, LIM>(s, a[g], b[g]);
+            }
+#pragma unroll
+            for (int u = 0; u < nh - G; ++u) {
+                wl[u] = wl[u + G];
+                wr[u] = wr[u + G];
+            }
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                wl[nh - G + g] = a[g];
+                wr[nh - G + g] = b[g];
+            }
+        }
+    } else {
+#pragma unroll
+        for (int v = 0; v < nh; ++v) {
+            double s[5];
+#pragma unroll
+            for (int o = -S; o <= S; ++o) {
+                s[2 + o] = centre[v * vstride + o * stride];
+            }
+            fast_reconstruct<REC, LIM>(s, wl[v], wr[v]);
+        }
+    }
+    double left[nh];
+#pragma unroll
+    for (int v = 0; v < nh; ++v) {
+        left[v] = __shfl_up_sync(0xffffffffu, wr[v], 1);
+    }
+    double f[nh];
+    const bool ok = fast_riemann<RS, NDIM>(gamma, gas, axis, left, wl, f);
+#pragma unroll
+    for (int v = 0; v < nh; ++v) {
+        const double fn = __shfl_down_sync(0xffffffffu, f[v], 1);
+        d[v] = f[v] - fn;
+    }
+    for (int t = 0; t < ntracer; ++t) {
+        double s[5];
+#pragma unroll
+        for (int o = -S; o <= S; ++o) {
+            s[2 + o] = centre[(nh + t) * vstride + o * stride];
+        }
+        double tl, tr;
+        fast_reconstruct<REC, LIM>(s, tl, tr);
+        const double tleft = __shfl_up_sync(0xffffffffu, tr, 1);
+        const double ft = (f[0] >= 0.0) ? f[0] * tleft : f[0] * tl;
+        const double fn = __shfl_down_sync(0xffffffffu, ft, 1);
+        d_tr[t] = ft - fn;
+    }
+    return ok;
+}
+
+// The sweep of one line by one warp: face_sweep's result. in_range
+// (warp-uniform): every value the line's stencils read is in range; a line
+// that is not, or whose face states are not, takes face_sweep's own code.
+template <int NDIM, int REC, int LIM, int RS, class T>
+__device__ __forceinline__ void sweep_line(const StageParams& p, bool in_range, const T* centre, int stride,
+                                           int vstride, T gamma, T gfac, int axis, T* d, T* d_tr) {
+    if constexpr (sizeof(T) == 8) {
+        constexpr int nh = 2 + NDIM;
+        bool redo = true;
+        if (in_range) {
+            redo = !fast_face_sweep<NDIM, REC, LIM, RS>(centre, stride, vstride, p.ntracer, p.gamma, p.gas, axis, d,
+                                                        d_tr);
+        }
+        if (__any_sync(0xffffffffu, redo)) {
+            double out[kMaxVars];
+            face_sweep_any<NDIM, REC, LIM, RS>(centre, stride, vstride, p.ntracer, gamma, gfac, axis, out);
+#pragma unroll
+            for (int v = 0; v < nh; ++v) {
+                d[v] = out[v];
+            }
+            for (int t = 0; t < p.ntracer; ++t) {
+                d_tr[t] = out[nh + t];
+            }
+        }
+    } else {
+        face_sweep<NDIM, REC, LIM, RS, T>(centre, stride, vstride, p.ntracer, gamma, gfac, axis, d, d_tr);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // 1D: one warp updates one segment of kTile cells, independently of the
 // other warps of its CTA (so one CTA can serve segments of different
@@ -502,16 +646,18 @@ __device__ __forceinline__ void segment1d(const StageParams& p, int x0, T* W, do
     constexpr int H = halo_of<REC>();
     constexpr int WN = seg1d_window<REC>();
     const int lane = threadIdx.x & 31;
+    bool in_range = p.gas.ok != 0;
     for (int it = lane; it < WN; it += 32) {
         const int i = p.ng + x0 - H + it;  // array index
         const bool inb = i >= 0 && i < p.xc;
-        flags |= load_prim<NDIM, T>(p, 0, 0, i, inb, W + it, WN);
+        flags |= load_prim<NDIM, T>(p, 0, 0, i, inb, W + it, WN, in_range);
     }
     __syncwarp();
+    in_range = __all_sync(0xffffffffu, in_range);
     const int cl = lane - 1;  // cell of this lane, relative to x0
     T d[nh], d_tr[kMaxVars];
     const T gfac = T((p.gamma + 1.0) / (2.0 * p.gamma));
-    face_sweep<NDIM, REC, LIM, RS, T>(W + H + cl, 1, WN, p.ntracer, T(p.gamma), gfac, 0, d, d_tr);
+    sweep_line<NDIM, REC, LIM, RS, T>(p, in_range, W + H + cl, 1, WN, T(p.gamma), gfac, 0, d, d_tr);
     __syncwarp();  // the window may be reloaded by the caller's next segment
 
     const double dt = stage_dt(p);
@@ -616,6 +762,7 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
     // phase 1: primitives of the tile and its cross-shaped halo
     constexpr int core = TY * WX;
     constexpr int items = core + 2 * H * TX;
+    bool in_range = p.gas.ok != 0;
     if constexpr (TMA) {
         // the box of WX x WY cells around the tile (x start even: the host
         // only takes this path when ng - H is even), all hydro variables;
@@ -659,7 +806,7 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
             const int j = p.ng + y0 + ty;
             const bool inb = i >= 0 && i < p.xc && j >= 0 && j < p.yc;
             flags |= staged_prim<NDIM, T>(p, stg + (ty + H) * WX + (tx + H), WX * WY, inb,
-                                          W + (ty + H) * P + (tx + H), WV);
+                                          W + (ty + H) * P + (tx + H), WV, in_range);
         }
     } else {
         for (int it = threadIdx.x; it < items; it += NT) {
@@ -676,10 +823,10 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
             const int i = p.ng + x0 + tx;
             const int j = p.ng + y0 + ty;
             const bool inb = i >= 0 && i < p.xc && j >= 0 && j < p.yc;
-            flags |= load_prim<NDIM, T>(p, k, j, i, inb, W + (ty + H) * P + (tx + H), WV);
+            flags |= load_prim<NDIM, T>(p, k, j, i, inb, W + (ty + H) * P + (tx + H), WV, in_range);
         }
     }
-    __syncthreads();
+    in_range = __syncthreads_and(in_range);
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -703,7 +850,7 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
         for (int line = warp; line < nlines; line += NW) {
             const T* centre = axis == 0 ? W + (line + H) * P + (c + H) : W + (c + H) * P + (line + H);
             T d[nh], d_tr[kMaxVars];
-            face_sweep<NDIM, REC, LIM, RS, T>(centre, axis == 0 ? 1 : P, WV, ntr, gamma, gfac, axis, d, d_tr);
+            sweep_line<NDIM, REC, LIM, RS, T>(p, in_range, centre, axis == 0 ? 1 : P, WV, gamma, gfac, axis, d, d_tr);
             const bool mine = lane >= 1 && lane <= kTile;
             if (axis == 1) {
                 if (mine) {
@@ -1034,6 +1181,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks2d)
     // phase 1: primitives of the tile and its halo rows
     // (TMA: column x of the tile is column x + xoff of the staged box)
     const int xoff = (p.ng + x0) & 1;
+    bool in_range = p.gas.ok != 0;
     if constexpr (TMA) {
         if (threadIdx.x == 0) {
             mbar_init(&mbar, 1);
@@ -1060,7 +1208,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks2d)
             const int x = it - r * kZCols;
             const int k = p.ng + z0 - H + r;
             const bool inb = x < vw && k >= 0 && k < p.zc;
-            flags |= staged_prim<NDIM, T>(p, stg + r * kZStageX + x + xoff, SV, inb, W + r * PZ + x, WV);
+            flags |= staged_prim<NDIM, T>(p, stg + r * kZStageX + x + xoff, SV, inb, W + r * PZ + x, WV,
+                                          in_range);
         }
     } else {
         for (int it = threadIdx.x; it < WZ * kZCols; it += kThreads) {
@@ -1069,10 +1218,10 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks2d)
             const int i = p.ng + x0 + x;
             const int k = p.ng + z0 - H + r;
             const bool inb = x < vw && k >= 0 && k < p.zc;
-            flags |= load_prim<NDIM, T>(p, k, j, i, inb, W + r * PZ + x, WV);
+            flags |= load_prim<NDIM, T>(p, k, j, i, inb, W + r * PZ + x, WV, in_range);
         }
     }
-    __syncthreads();
+    in_range = __syncthreads_and(in_range);
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -1087,7 +1236,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks2d)
     for (int col = warp; col < vw; col += kWarps) {
         T* centre = W + (c + H) * PZ + col;
         T d[nh], d_tr[kMaxVars];
-        face_sweep<NDIM, REC, LIM, RS, T>(centre, PZ, WV, ntr, gamma, gfac, 2, d, d_tr);
+        sweep_line<NDIM, REC, LIM, RS, T>(p, in_range, centre, PZ, WV, gamma, gfac, 2, d, d_tr);
         __syncwarp();
         if (lane >= 1 && lane <= TZ) {
 #pragma unroll

@@ -159,7 +159,22 @@ __global__ void __launch_bounds__(256) cons_to_prim_kernel(StageParams p, double
     }
 }
 
+// The quotients, reciprocals and roots of exact_fp64.cuh by themselves.
+__global__ void __launch_bounds__(256) exact_ops_kernel(int op, const double* a, const double* b, double* out,
+                                                        long long n) {
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
+         k += (long long)gridDim.x * blockDim.x) {
+        out[k] = op == 0 ? exact_div(a[k], b[k]) : op == 1 ? exact_rcp(a[k]) : exact_sqrt(a[k]);
+    }
+}
+
 } // namespace
+
+cudaError_t launch_exact_ops(int op, const double* a, const double* b, double* out, long long n, cudaStream_t s) {
+    const int blocks = (int)(n < 148LL * 8 * 256 ? cdiv(n, 256) : 148 * 8);
+    exact_ops_kernel<<<blocks, 256, 0, s>>>(op, a, b, out, n);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_cons_to_prim(const StageParams& p, double* w, int ndim, cudaStream_t s) {
     const int blocks = (int)(p.plane < 148LL * 8 * 256 ? cdiv(p.plane, 256) : 148 * 8);
