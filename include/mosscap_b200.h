@@ -483,10 +483,10 @@ int64_t mc_launch_count(const mc_ctx* ctx);
  * be measured. No counterpart in the reference. */
 mc_status mc_debug_reverse_reciprocal(const double* x, double* out, int64_t n, void* stream);
 
-/* Diagnostic: the branch-free quotient (op 0: out[i] = a[i] / b[i]), reciprocal
- * (op 1: 1 / a[i]) and root (op 2: sqrt(a[i])) of the FP64 stage kernels, on
- * device arrays of n doubles (b is read by op 0 only), so that their rounding can
- * be compared with IEEE arithmetic. No counterpart in the reference. */
+/* Diagnostic: the branch-free quotient (op 0: out[i] = a[i] / b[i]) and root
+ * (op 1: sqrt(a[i]); b unused) of the FP64 stage kernels, on device arrays of
+ * n doubles, so that their rounding can be compared with IEEE arithmetic. No
+ * counterpart in the reference. */
 mc_status mc_debug_exact_ops(int32_t op, const double* a, const double* b, double* out, int64_t n, void* stream);
 
 /* Message of the last failed call on this thread (static storage). */

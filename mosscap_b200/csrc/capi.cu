@@ -1243,7 +1243,7 @@ mc_status mc_stage_time(mc_ctx* c, int32_t kind, double* total_ms, int64_t* laun
 }
 
 mc_status mc_debug_exact_ops(int32_t op, const double* a, const double* b, double* out, int64_t n, void* stream) {
-    if (!a || !out || n < 0 || op < 0 || op > 2 || (op == 0 && !b)) {
+    if (!a || !out || n < 0 || op < 0 || op > 1 || (op == 0 && !b)) {
         return fail(MC_ERR_INVALID_ARGUMENT, "null argument, negative count or unknown op");
     }
     if (n > 0) {

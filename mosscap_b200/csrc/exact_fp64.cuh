@@ -9,44 +9,60 @@
 // quotients are in flight, since nothing moves across the branch. The forms here
 // are straight-line code for operands whose exponents were checked
 // beforehand, once per cell (the range tests below) instead of once per
-// quotient: 9 FP64 instructions per quotient, 5 for a further quotient with
+// quotient: 7 FP64 instructions per quotient, 5 for a further quotient with
 // the same denominator, 8 per root, all of them free to overlap.
 //
 // Where a product with a power of two feeds an addition the two are written
 // as one fma: the product is exact, so the result is the same rounding of the
 // same sum as in physics.cuh. Everything else keeps the order of
 // physics.cuh, whose functions are evaluated instead (generic form) wherever
-// a range test fails. Measured (B200, two steps, bit-identical): KH 2048^2 WENO5-Z
-// + HLLC 3.76 -> 3.16 ms, KH 256^2 (8 steps) 1.05 -> 0.80 ms, 384 MUSCL + HLLC
-// problems (4 steps) 10.4 -> 9.5 ms.
+// a range test fails.
 //
-// Division (Markstein, IBM J. Res. Dev. 34, 1990; Cornea, Harrison and Tang,
-// "Scientific Computing on Itanium-based Systems", 2002): the seed
-// rcp.approx.ftz.f64 (relative error <= 2^-19.9 over all of its inputs,
-// measured; it reads the operand's upper word only) is refined by two
-// Newton steps to y2 = RN((1/b)(1 + z)), |z| <= 2^-79; the quotient is corrected
-// once with the half-refined reciprocal, which leaves it within
-// (1/2 + 2^-26) ulp of a/b, and once more with y2, where the residual is exact.
-// The last rounding could only differ from RN(a/b) if a/b lay within
-// ulp/2 * |y2 b - 1| of a rounding boundary. For 53-bit integers A, B (the
-// operands' significands) a quotient that is not on one is at least 1/(2B) ulp
-// away from it, so that needs B > 2^53 (1 - 2^-27) and 1/b within |z| of a
-// rounding boundary of its own. For those B the seed is the same, 1/2 exactly
-// (scaled), the first step leaves an error below 2^-53 and the second |z| <= 2^-105,
-// which leaves B = 2^53 - 1 alone (M = 2^53 + 1, M B = 2^106 - 1): its reciprocal
-// lies just above a boundary and y2 on it, where rounding to even goes down. The
-// lowest bit of e1 is set for that one (2^-52 of a correction that is itself
-// below 2^-39). Tested on the closest quotients of every B = 2^53 - k, odd
-// k < 2^15 (tests/test_exact_ops_gpu.py).
+// What an FP64 instruction costs (measured, 20 warps per SM): two cycles of an SM
+// sub-partition for products, sums and fmas that read at most two distinct registers
+// (a constant or a repeated operand as the third), three for an fma of three
+// registers. So the refinements prefer the forms 1 - b y, e + e e and t + t s.
+// With the sweeps' code as it is these cycles are what bounds them (2D WENO5-Z).
 //
-// Square root (same sources; Cornea-Hasegan, Golliver and Markstein, ARITH-14,
-// 1999, for the enumeration of the hard cases): seed rsqrt.approx.ftz.f64
+// Division. With the seed y = (1/b)(1 - e) and s = e + e^2, (1/b) = y (1 + s) up to a
+// factor 1 + e^3. q = t + t s with t = a y is within 1.02 ulp of a/b (t's
+// rounding, its own, e^3 <= 2^-59.8), the residual d = b q - a is exact, and the
+// result q - (d + d s) y is a/b rounded once, but for an error of c = d / b of
+// relatively 2^-53 / m + 2^-59.8, m in [1, 2) the significand of d + d s, b's up to
+// 2^-19.9. That can only matter for a/b near a rounding boundary, where |c| is half an ulp.
+// With 53-bit integers A, B as the operands' significands a quotient is at least
+// 1 / (2B) ulp away from a boundary (it cannot lie on one), that is 2^-53 / b ulp,
+// and the error is (2^-54 / b) (1 + 2^-5.8) ulp: about half of it. (Markstein, IBM J.
+// Res. Dev. 34, 1990, has the correction by an exact residual, and this way of
+// bounding it.) Two things need a closer look. For b within 2^-26 of 2, B = 2^53 - k, the
+// seed is 1/2 exactly and d + d s can pass the next power of two, where m is 1: for
+// the closest quotient it lies k 2^-54 units above the middle between two doubles, and
+// the rounding of s moves it by less than that unless k = 1, where by as much; s is
+// therefore rounded up, which settles 1 / (2 - 2^-52). And for q a power of two and
+// a/b below it, where an ulp is half as long, a boundary is also at three quarters of q's
+// ulp (the one at a quarter is out of reach, a/b = 1 - n/B with integer n): n = 1 and B
+// next to 2^54 / 3, two quotients. Both kinds are tested with the closest quotients of
+// many other B (tests/test_exact_ops_gpu.py).
+//
+// The seed rcp.approx.ftz.f64 has a relative error <= 2^-19.93 over all of its
+// inputs (it reads the operand's upper word only; measured over all of them).
+//
+// Square root (Cornea-Hasegan, Golliver and Markstein, ARITH-14, 1999, for the
+// form and the enumeration of the hard cases): seed rsqrt.approx.ftz.f64
 // (<= 2^-20.0), one third-order step for root and half reciprocal, one exact
 // residual. The value before the last rounding is within 2^-102.8 of the root of
 // x in [1, 4); a root at odd distance j from a rounding boundary, in units where
 // the boundary's square is an integer, is at least j 2^-108 from it, so only
-// j <= 37 can round differently; all significands with j < 64 are tested.
+// j <= 37 can round differently; all significands with j < 256 are tested.
+//
+// Measured (B200, KH 2048^2 WENO5-Z + HLLC, one stage, bit-identical): IEEE division and
+// root 0.594 ms; quotients by two Newton steps and two corrections (nine instructions)
+// 0.506 ms; this form 0.453 ms. Six instructions without d s, a test of d against
+// half an ulp (four integer instructions) and the lines where it fires
+// evaluated again: 0.514 ms, the test alone 0.038 ms.
 #pragma once
+
+#include <cmath>
 
 #include "physics.cuh"
 
@@ -63,40 +79,31 @@ __device__ __forceinline__ double rsqrt_seed(double x) {
     return r;
 }
 
-// 1 / b for exact_quot: y1 within 2^-39 of it, y2 within an ulp.
+// A denominator: y = (1/b)(1 - e), s = e + e^2.
 struct Recip {
-    double b, y1, y2;
+    double b, y, s;
 };
 __device__ __forceinline__ Recip recip_of(double b) {
     Recip r;
     r.b = b;
-    const double y0 = rcp_seed(b);
-    const double e0 = fma(-b, y0, 1.0);
-    r.y1 = fma(y0, e0, y0);
-    double e1 = fma(-b, r.y1, 1.0);
-    e1 = __hiloint2double(__double2hiint(e1), __double2loint(e1) | 1);
-    r.y2 = fma(r.y1, e1, r.y1);
+    r.y = rcp_seed(b);
+    const double e = fma(-b, r.y, 1.0);
+    r.s = __fma_ru(e, e, e);
     return r;
 }
 
-// RN(a / b) for b whose reciprocal is normal, and a that is zero (b > 0 then:
-// the residuals are formed as b q - a, which keeps the zero's sign) or so that
-// the quotient is normal and |a| > 2^-900.
+// RN(a / b) for b whose reciprocal is normal and a that is zero (the result is a
+// zero of either sign: no result of the stage kernels depends on it) or so
+// that the quotient is normal and |a| > 2^-900.
 __device__ __forceinline__ double exact_quot(double a, const Recip& r) {
-    double q = __dmul_rn(a, r.y1);
+    const double t = __dmul_rn(a, r.y);
+    const double q = fma(t, r.s, t);
     double d = fma(r.b, q, -a);
-    q = fma(-d, r.y1, q);
-    d = fma(r.b, q, -a);
-    return fma(-d, r.y2, q);
+    d = fma(d, r.s, d);
+    return fma(-d, r.y, q);
 }
 __device__ __forceinline__ double exact_div(double a, double b) {
     return exact_quot(a, recip_of(b));
-}
-// RN(1 / b)
-__device__ __forceinline__ double exact_rcp(double b) {
-    const Recip r = recip_of(b);
-    const double d = fma(b, r.y2, -1.0);
-    return fma(-d, r.y2, r.y2);
 }
 
 // RN(sqrt(x)) for x in [2^-900, 2^900]. Anything else gives no such value and
@@ -139,15 +146,16 @@ __device__ __forceinline__ bool in_range_pos4(double a, double b, double c, doub
 // The constants of the gas of one launch, formed on the host (kernel
 // parameters: constant-bank operands, no registers).
 struct FastGas {
-    double gm1, gfac;  // gamma - 1, (gamma + 1) / (2 gamma)
-    double rgm1;       // RN(1 / (gamma - 1))
-    int ok;            // gamma and gamma - 1 in [2^-20, 2^20]
+    double gm1, gfac;    // gamma - 1, (gamma + 1) / (2 gamma)
+    double rgm1, sgm1;   // RN(1 / (gamma - 1)) and its residual (Recip's y and s)
+    int ok;              // gamma and gamma - 1 in [2^-20, 2^20]
 };
 inline FastGas fast_gas(double gamma) {
     FastGas g;
     g.gm1 = gamma - 1.0;
     g.gfac = (gamma + 1.0) / (2.0 * gamma);
     g.rgm1 = 1.0 / g.gm1;
+    g.sgm1 = std::fma(-g.gm1, g.rgm1, 1.0);
     g.ok = gamma <= 0x1p20 && g.gm1 >= 0x1p-20 ? 1 : 0;
     return g;
 }
@@ -159,18 +167,16 @@ template <int NDIM>
 __device__ __forceinline__ bool fast_prim(double gm1, const double* q, double* w) {
     const Recip r = recip_of(q[0]);
     w[0] = q[0];
-    w[1] = exact_quot(q[1], r);
-    bool ok = in_range_pos(q[0]) && in_range_any(w[1]);
-    double v2 = __dmul_rn(w[1], w[1]);
-    if constexpr (NDIM > 1) {
-        w[2] = exact_quot(q[2], r);
-        v2 = __dadd_rn(v2, __dmul_rn(w[2], w[2]));
-        ok = ok && in_range_any(w[2]);
+#pragma unroll
+    for (int d = 1; d <= NDIM; ++d) {
+        w[d] = exact_quot(q[d], r);
     }
-    if constexpr (NDIM > 2) {
-        w[3] = exact_quot(q[3], r);
-        v2 = __dadd_rn(v2, __dmul_rn(w[3], w[3]));
-        ok = ok && in_range_any(w[3]);
+    bool ok = in_range_pos(q[0]);
+    double v2 = 0.0;
+#pragma unroll
+    for (int d = 1; d <= NDIM; ++d) {
+        ok = ok && in_range_any(w[d]);
+        v2 = d == 1 ? __dmul_rn(w[d], w[d]) : __dadd_rn(v2, __dmul_rn(w[d], w[d]));
     }
     // E - (0.5 rho) v2: the factor 1/2 is exact
     w[1 + NDIM] = __dmul_rn(gm1, fma(-0.5, __dmul_rn(q[0], v2), q[1 + NDIM]));
@@ -307,21 +313,16 @@ __device__ __forceinline__ bool fast_riemann(double gamma, const FastGas& gas, i
     bool ok = in_range_pos4(wL[0], wR[0], pL, pR);
     const double csL = exact_sqrt(exact_div(gamma * pL, wL[0]));
     const double csR = exact_sqrt(exact_div(gamma * pR, wR[0]));
-    // cons_from_prim: momenta and total energy (0.5 rho v^2 with an exact 1/2)
-    double qL[nh], qR[nh];
-    double kL = 0.0, kR = 0.0;
-    qL[0] = wL[0];
-    qR[0] = wR[0];
+    const Recip rg{gas.gm1, gas.rgm1, gas.sgm1};
+    // total energy of a state (0.5 rho v^2 with an exact 1/2)
+    auto energy = [&](const double* w) {
+        double k = w[1] * w[1];
 #pragma unroll
-    for (int d = 1; d <= NDIM; ++d) {
-        qL[d] = wL[0] * wL[d];
-        qR[d] = wR[0] * wR[d];
-        kL = d == 1 ? wL[d] * wL[d] : kL + wL[d] * wL[d];
-        kR = d == 1 ? wR[d] * wR[d] : kR + wR[d] * wR[d];
-    }
-    const Recip rg{gas.gm1, gas.rgm1, gas.rgm1};
-    qL[ie] = fma(0.5, wL[0] * kL, exact_quot(pL, rg));
-    qR[ie] = fma(0.5, wR[0] * kR, exact_quot(pR, rg));
+        for (int d = 2; d <= NDIM; ++d) {
+            k += w[d] * w[d];
+        }
+        return fma(0.5, w[0] * k, exact_quot(w[ie], rg));
+    };
     if constexpr (RS == kHllc) {
         const double cs2 = csL + csR, rho2 = wL[0] + wR[0];
         // (vL - vR) rho_avg cs_avg with both factors 1/2 taken out (exact)
@@ -335,38 +336,41 @@ __device__ __forceinline__ bool fast_riemann(double gamma, const FastGas& gas, i
         const double aR = vR + csR * cRstar;
         const double bM = smin(-tiny, aL);
         const double bP = smax(tiny, aR);
-        double vxL = vL - aL;
-        double vxR = vR - aR;
-        const double tL = pL + vxL * along<NDIM>(qL, axis);
-        const double tR = pR + vxR * along<NDIM>(qR, axis);
+        const double vxL = vL - aL;
+        const double vxR = vR - aR;
+        const double tL = pL + vxL * (wL[0] * vL);
+        const double tR = pR + vxR * (wR[0] * vR);
         const double mL = wL[0] * vxL;
         const double mR = -(wR[0] * vxR);
         const Recip rm = recip_of(mL + mR);
         const double aM = exact_quot(tL - tR, rm);
         const double cp = smax(exact_quot(mL * tR + mR * tL, rm), 0.0);
-        // the upwind side only: the other's flux has weight zero. For finite g
-        // s f + 0 g is s f, but for the sign of a zero, and no result depends on
-        // that: every flux difference is added to a sum that starts from +0
         const bool left = aM >= 0.0;
         const double den = left ? (aM - bM) : (bP - aM);
         const Recip rd = recip_of(den);
         const double s_out = exact_quot(left ? aM : -aM, rd);
         const double sM = exact_quot(left ? -bM : bP, rd);
         // the wave-speed differences, like the face states, must be ordinary numbers
-        ok = ok && in_range_pos4(mL + mR, den, mL + mR, den);
-        const double w0 = left ? wL[0] : wR[0];
-        const double vx = left ? vL - bM : vR - bP;
-        const double p = left ? pL : pR;
+        ok = ok && in_range_pos(rm.b) && in_range_pos(den);
+        // the upwind side only: the other's flux has weight zero. For finite g
+        // s f + 0 g is s f, but for the sign of a zero, and no result depends on
+        // that: every flux difference is added to a sum that starts from +0
+        double w[nh];
+#pragma unroll
+        for (int i = 0; i < nh; ++i) {
+            w[i] = left ? wL[i] : wR[i];
+        }
         const double v = left ? vL : vR;
-        const double mf = w0 * vx;
+        const double vx = v - (left ? bM : bP);
+        const double mf = w[0] * vx;
         double f[nh];
         f[0] = mf;
 #pragma unroll
         for (int d = 1; d <= NDIM; ++d) {
-            f[d] = mf * (left ? wL[d] : wR[d]);
+            f[d] = mf * w[d];
         }
-        add_along<NDIM>(f, axis, p);
-        f[ie] = (left ? qL[ie] : qR[ie]) * vx + p * v;
+        add_along<NDIM>(f, axis, w[ie]);
+        f[ie] = energy(w) * vx + w[ie] * v;
 #pragma unroll
         for (int i = 0; i < nh; ++i) {
             flux[i] = s_out * f[i];
@@ -374,8 +378,17 @@ __device__ __forceinline__ bool fast_riemann(double gamma, const FastGas& gas, i
         add_along<NDIM>(flux, axis, sM * cp);
         flux[ie] += sM * cp * aM;
     } else {
-        // flux_from_prim with cons_from_prim's total energy (the same sum)
-        double fL[nh], fR[nh];
+        // momenta and energies; flux_from_prim's total energy is the same sum
+        double qL[nh], qR[nh], fL[nh], fR[nh];
+        qL[0] = wL[0];
+        qR[0] = wR[0];
+#pragma unroll
+        for (int d = 1; d <= NDIM; ++d) {
+            qL[d] = wL[0] * wL[d];
+            qR[d] = wR[0] * wR[d];
+        }
+        qL[ie] = energy(wL);
+        qR[ie] = energy(wR);
         const double mfL = wL[0] * vL, mfR = wR[0] * vR;
         fL[0] = mfL;
         fR[0] = mfR;
@@ -399,7 +412,7 @@ __device__ __forceinline__ bool fast_riemann(double gamma, const FastGas& gas, i
             const double sR = smax(-tiny, smax(vL + csL, vL + csR));
             const double den = sR - sL;
             ok = ok && in_range_pos(den);
-            const double sM = exact_rcp(den);
+            const double sM = exact_div(1.0, den);
 #pragma unroll
             for (int i = 0; i < nh; ++i) {
                 flux[i] = sM * (sR * fL[i] - sL * fR[i] + sR * sL * (qR[i] - qL[i]));

@@ -56,7 +56,7 @@ cudaError_t launch_fill_bcs(const StageParams& p, int ndim, cudaStream_t s);
 // Primitives of p.q_in over every cell (ghosts included) into w, tracers
 // as mass fractions.
 cudaError_t launch_cons_to_prim(const StageParams& p, double* w, int ndim, cudaStream_t s);
-// The quotients (op 0), reciprocals (1) and roots (2) of exact_fp64.cuh.
+// The quotients (op 0) and roots (1) of exact_fp64.cuh.
 cudaError_t launch_exact_ops(int op, const double* a, const double* b, double* out, long long n, cudaStream_t s);
 // CFL minimum over every cell of Q (ghosts included) into blk->cfl_min_bits,
 // which the launch first resets.

@@ -159,12 +159,12 @@ __global__ void __launch_bounds__(256) cons_to_prim_kernel(StageParams p, double
     }
 }
 
-// The quotients, reciprocals and roots of exact_fp64.cuh by themselves.
+// The quotients (op 0) and roots (op 1) of exact_fp64.cuh by themselves.
 __global__ void __launch_bounds__(256) exact_ops_kernel(int op, const double* a, const double* b, double* out,
                                                         long long n) {
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
          k += (long long)gridDim.x * blockDim.x) {
-        out[k] = op == 0 ? exact_div(a[k], b[k]) : op == 1 ? exact_rcp(a[k]) : exact_sqrt(a[k]);
+        out[k] = op == 0 ? exact_div(a[k], b[k]) : exact_sqrt(a[k]);
     }
 }
 

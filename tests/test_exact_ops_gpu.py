@@ -32,14 +32,15 @@ def _run(lib, op, a, b=None):
 
 
 def _same(got, want):
+    got, want = got + 0.0, want + 0.0
     bad = np.flatnonzero(got.view(np.uint64) != want.view(np.uint64))
     assert bad.size == 0, (bad.size, bad[:4], got[bad[:4]], want[bad[:4]])
 
 
 def _hard_quotients():
     """(a, b) in [1, 2) with a / b < 1 at the least distance from a rounding
-    boundary, 2^54 A - M B = +-1 with odd M: for b just below 2 (where the
-    reciprocal itself may be one bit off) and for random b."""
+    boundary, 2^54 A - M B = +-1 with odd M: for b just below 2 and for random b;
+    and a / b = 1 - 1 / B next to 1 - 3 2^-54."""
     rng = np.random.default_rng(1)
     bs = [2 ** 53 - k for k in range(1, 1 << 15, 2)] + [int(x) | 1 for x in rng.integers(2 ** 52, 2 ** 53, 20000)]
     out = []
@@ -51,6 +52,8 @@ def _hard_quotients():
             assert (A << 54) - M * B == j
             if M >= 1 << 53 and A >= 1 << 52:
                 out.append((A, B))
+    B = (1 << 54) // 3
+    out += [(B - 1, B), (B, B + 1)]
     a = np.array([x for x, _ in out], dtype=np.float64) * 2.0 ** -52
     return a, np.array([y for _, y in out], dtype=np.float64) * 2.0 ** -52
 
@@ -61,15 +64,15 @@ def test_quotients_equal_ieee_division(gpu_lib):
     b = rng.uniform(1.0, 2.0, n) * 2.0 ** rng.integers(-120, 121, n)
     a = rng.uniform(1.0, 2.0, n) * 2.0 ** rng.integers(-250, 251, n) * rng.choice([-1.0, 1.0], n)
     a[: n // 16] = b[: n // 16] * rng.integers(1, 1 << 20, n // 16)  # near and at exact quotients
-    a[-8:] = [0.0, -0.0] * 4
+    a[-8:] = [0.0, -0.0] * 4  # (compared as values: the sign of a zero is free)
     b[:6] = [1.0, np.nextafter(2.0, 1.0), np.nextafter(1.0, 2.0), 3.0, 0.4, 2.0 / 3.0]
     _same(_run(gpu_lib, 0, a, b), a / b)
-    _same(_run(gpu_lib, 1, b), 1.0 / b)
+    _same(_run(gpu_lib, 0, np.ones_like(b), b), 1.0 / b)
     a, b = _hard_quotients()
     assert a.size > 10000
     _same(_run(gpu_lib, 0, a, b), a / b)
     _same(_run(gpu_lib, 0, -a * 2.0 ** 200, b * 2.0 ** -60), -a / b * 2.0 ** 260)
-    _same(_run(gpu_lib, 1, b), 1.0 / b)
+    _same(_run(gpu_lib, 0, np.ones_like(b), b), 1.0 / b)
 
 
 def _square_roots_mod(c, bits):
@@ -89,7 +92,7 @@ def test_roots_equal_ieee_square_root(gpu_lib):
     x = rng.uniform(1.0, 4.0, n) * 4.0 ** rng.integers(-250, 251, n)
     x[: n // 16] = rng.integers(1, 1 << 26, n // 16).astype(np.float64) ** 2  # exact roots
     x[:4] = [1.0, np.nextafter(1.0, 2.0), np.nextafter(4.0, 1.0), 2.0]
-    _same(_run(gpu_lib, 2, x), np.sqrt(x))
+    _same(_run(gpu_lib, 1, x), np.sqrt(x))
     # x = (M^2 + j) 2^-106 with odd M (a rounding boundary of the root) and odd j
     hard = []
     for bits, scale in ((54, 2.0 ** -52), (55, 2.0 ** -51)):  # x in [1, 2), x in [2, 4)
@@ -106,7 +109,7 @@ def test_roots_equal_ieee_square_root(gpu_lib):
     hard = np.array(hard)
     assert hard.size > 0
     for k in (0, 1, -100, 101):
-        _same(_run(gpu_lib, 2, hard * 4.0 ** k), np.sqrt(hard * 4.0 ** k))
+        _same(_run(gpu_lib, 1, hard * 4.0 ** k), np.sqrt(hard * 4.0 ** k))
 
 
 def _state(nd, n, kind, seed, nt):
