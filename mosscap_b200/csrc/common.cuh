@@ -71,6 +71,7 @@ struct StageParams {
     // tile_rows, if nonzero, is the launch's grid height. All zero: every
     // tile row, one per blockIdx.y.
     int row_split, row_skip, tile_rows;
+    int tile_h;                       // 2D, LOW kernels: rows of a tile (at most kTile)
 };
 
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;

@@ -52,34 +52,58 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
 
 // The TMA tile load applies when the kernel has a TMA form for this
 // reconstruction and still fits its CTAs per SM, the tile's x start is even
-// (ng - H even), there are no tracers, and the stage input's tensor map can
-// be built (16-byte aligned base, even row length, box inside the array).
+// (ng - H even, or the staged tile has MUSCL's spare columns), there are no
+// tracers, and the stage input's tensor map can be built (16-byte aligned
+// base, even row length, box inside the array).
 template <int NDIM, int REC>
 bool use_tma(const StageParams& p, CUtensorMap* map) {
+    const int th = p.tile_h ? p.tile_h : kTile;
     using G = TileGeom<2, REC>;
-    if (!tma_capable<NDIM, REC, Real>(p.nvar) || p.ntracer != 0 || ((p.ng - G::H) & 1) != 0) {
+    if (!tma_capable<NDIM, REC, Real>(p.nvar) || p.ntracer != 0 || (((p.ng - G::H) & 1) != 0 && G::SX == G::WX)) {
         return false;
     }
     std::memset(map, 0, sizeof(*map));
-    return tma_map_for(p.q_in, p.xc, p.yc, p.zc, p.nvar, G::WX, G::WY, 2 + NDIM, map);
+    return tma_map_for(p.q_in, p.xc, p.yc, p.zc, p.nvar, G::SX, th + 2 * G::H, 2 + NDIM, map);
+}
+
+// 2D grids that leave SMs without a tile of kTile rows: the rows of a lower tile
+// (8 at least) with which the grid still has at most one tile per SM, or 0 where even
+// the full height has more. One tile per SM leaves its time to the latency of the
+// lines its warps sweep one after the other: fewer lines per tile, and 16 warps
+// instead of 10 (LOW kernels). Measured per stage (FP64 WENO5-Z + HLLC, cold L2): 256^2
+// 32.7 -> 22.5 us (16 rows; 26.6 with them in the regular kernel, 27.5 in the LOW kernel
+// with 30), 128^2 30.7 -> 20.4 us; MUSCL 256^2 24.6 -> 16.4 us, FP32 256^2 23.5 -> 15.4 us.
+// With more than one tile per SM the regular kernel is faster (512^2: 53 - 55 us with 22
+// or 30 rows, 59 in the LOW kernel).
+constexpr int kSMs = 148;
+inline int low_tile_rows(int nx, int ny) {
+    const int columns = cdiv(nx, kTile);
+    if (columns * cdiv(ny, kTile) > kSMs) {
+        return 0;
+    }
+    int th = kTile;
+    while (th > 8 && columns * cdiv(ny, th - 1) <= kSMs) {
+        --th;
+    }
+    return th;
 }
 
 // The tiled kernel (2D stage, or the 3D x-y plane pass) with or without the
 // TMA tile load.
-template <int NDIM, int REC, int LIM, int RS, bool SRC, bool TMA>
+template <int NDIM, int REC, int LIM, int RS, bool SRC, bool TMA, bool LOW = false>
 cudaError_t launch_tiled(const StageParams& p, const CUtensorMap& map, cudaStream_t s) {
     if constexpr (TMA && !tma_capable<NDIM, REC, Real>(2 + NDIM)) {
         return cudaErrorNotSupported;  // never taken: use_tma refused it
     } else {
-        auto k = stage2d_kernel<NDIM, REC, LIM, RS, Real, SRC, TMA, (NDIM == 2 && MC_DEFER != 0)>;
+        auto k = stage2d_kernel<NDIM, REC, LIM, RS, Real, SRC, TMA, (NDIM == 2 && MC_DEFER != 0), LOW>;
         const size_t sm = TMA ? smem_bytes_tma<NDIM, REC, Real>(p.nvar) : smem_bytes<NDIM, REC, Real>(p.nvar);
         cudaError_t e = allow_smem(k, sm);
         if (e != cudaSuccess) {
             return e;
         }
-        const int rows = (NDIM == 2 && p.tile_rows > 0) ? p.tile_rows : cdiv(p.ny, kTile);
+        const int rows = (NDIM == 2 && p.tile_rows > 0) ? p.tile_rows : cdiv(p.ny, LOW ? p.tile_h : kTile);
         const dim3 grid(cdiv(p.nx, kTile), rows, NDIM == 3 ? p.nz : 1);
-        k<<<grid, dim3(tile_threads<NDIM, Real>()), sm, s>>>(p, map);
+        k<<<grid, dim3(tile_threads<NDIM, Real, LOW>()), sm, s>>>(p, map);
         return cudaGetLastError();
     }
 }
@@ -124,6 +148,14 @@ cudaError_t launch_one(const StageParams& p, int pass, cudaStream_t s) {
 #elif MC_DIM == 2
     (void)pass;
     CUtensorMap map;
+#if !MC_DEFER
+    if (const int th = p.tile_rows == 0 ? low_tile_rows(p.nx, p.ny) : 0) {
+        StageParams t = p;
+        t.tile_h = th;
+        return use_tma<2, REC>(t, &map) ? launch_tiled<2, REC, LIM, RS, MC_SRC, true, true>(t, map, s)
+                                        : launch_tiled<2, REC, LIM, RS, MC_SRC, false, true>(t, map, s);
+    }
+#endif
     if (use_tma<2, REC>(p, &map)) {
         return launch_tiled<2, REC, LIM, RS, MC_SRC, true>(p, map, s);
     }

@@ -48,6 +48,7 @@ struct TileGeom {
     static constexpr int TX = kTile;
     static constexpr int TY = NDIM == 1 ? 1 : kTile;
     static constexpr int WX = TX + 2 * H;                    // stored columns
+    static constexpr int SX = WX + (H == 2 ? 2 : 0);         // staged columns (TMA): from the even one before
     static constexpr int P = (WX % 2 == 0) ? WX + 1 : WX;    // odd pitch: conflict-free columns
     static constexpr int WY = NDIM == 1 ? 1 : TY + 2 * H;    // stored rows
     static constexpr int PY = TX + 1;                        // odd pitch of the y divergence
@@ -72,19 +73,28 @@ __host__ __device__ constexpr size_t smem_bytes(int nvar) {
 
 // Shared memory of the tiled kernels with a TMA tile load: a 128-byte
 // aligned region that first holds the conserved tile as the TMA copies it
-// (WY rows x WX cells x 2 + NDIM variables, doubles; corners included) and
+// (WY rows x SX cells x 2 + NDIM variables, doubles; corners included) and
 // later the y divergences (it is free once the tile is converted), then the
 // primitive tile W.
 template <int NDIM, int REC>
 __host__ __device__ constexpr size_t tma_stage_bytes() {
     using G = TileGeom<2, REC>;
-    return sizeof(double) * (size_t)(2 + NDIM) * G::WY * G::WX;
+    return sizeof(double) * (size_t)(2 + NDIM) * G::WY * G::SX;
+}
+// Whether the staged tile outlives the conversion (2D, FP64; FP32 MUSCL and FOG):
+// the y divergences then lie after it, and the finishing takes each
+// cell's stage input from it.
+// Shared memory still allows two CTAs per SM (FP32 three). Measured with the stage input
+// from L2 -> from the staged tile: KH 2048^2 stage 0.451 -> 0.444 ms, PPM + HLL 0.336 -> 0.332.
+template <int NDIM, int REC, class T>
+__host__ __device__ constexpr bool keeps_stage() {
+    return NDIM == 2 && (sizeof(T) == 8 || halo_of<REC>() < 3);
 }
 template <int NDIM, int REC, class T>
 __host__ __device__ constexpr size_t tma_region_bytes(int nvar) {
     const size_t dy = sizeof(T) * (size_t)nvar * smem_dqy_per_var<2, REC>();
     const size_t st = tma_stage_bytes<NDIM, REC>();
-    return ((dy > st ? dy : st) + 127) / 128 * 128;
+    return ((keeps_stage<NDIM, REC, T>() ? dy + st : dy > st ? dy : st) + 127) / 128 * 128;
 }
 template <int NDIM, int REC, class T>
 __host__ __device__ constexpr size_t smem_bytes_tma(int nvar) {
@@ -598,11 +608,12 @@ __device__ __forceinline__ bool fast_face_sweep(const double* centre, int stride
 }
 
 // The sweep of one line by one warp: face_sweep's result. in_range
-// (warp-uniform): every value the line's stencils read is in range; a line
+// (warp-uniform): every value the line's stencils read is in range; cells: the
+// number of cells from lane 1 on whose divergence is wanted; a line
 // that is not, or whose face states are not, takes face_sweep's own code.
 template <int NDIM, int REC, int LIM, int RS, class T>
-__device__ __forceinline__ void sweep_line(const StageParams& p, bool in_range, const T* centre, int stride,
-                                           int vstride, T gamma, T gfac, int axis, T* d, T* d_tr) {
+__device__ __forceinline__ void sweep_line(const StageParams& p, bool in_range, int cells, const T* centre,
+                                           int stride, int vstride, T gamma, T gfac, int axis, T* d, T* d_tr) {
     if constexpr (sizeof(T) == 8) {
         constexpr int nh = 2 + NDIM;
         bool redo = true;
@@ -610,7 +621,9 @@ __device__ __forceinline__ void sweep_line(const StageParams& p, bool in_range, 
             redo = !fast_face_sweep<NDIM, REC, LIM, RS>(centre, stride, vstride, p.ntracer, p.gamma, p.gas, axis, d,
                                                         d_tr);
         }
-        if (__any_sync(0xffffffffu, redo)) {
+        // only the faces of the line's cells count: lanes 1 .. cells + 1
+        const int lane = threadIdx.x & 31;
+        if (__any_sync(0xffffffffu, redo && lane >= 1 && lane <= cells + 1)) {
             double out[kMaxVars];
             face_sweep_any<NDIM, REC, LIM, RS>(centre, stride, vstride, p.ntracer, gamma, gfac, axis, out);
 #pragma unroll
@@ -657,7 +670,7 @@ __device__ __forceinline__ void segment1d(const StageParams& p, int x0, T* W, do
     const int cl = lane - 1;  // cell of this lane, relative to x0
     T d[nh], d_tr[kMaxVars];
     const T gfac = T((p.gamma + 1.0) / (2.0 * p.gamma));
-    sweep_line<NDIM, REC, LIM, RS, T>(p, in_range, W + H + cl, 1, WN, T(p.gamma), gfac, 0, d, d_tr);
+    sweep_line<NDIM, REC, LIM, RS, T>(p, in_range, min(kTile, p.nx - x0), W + H + cl, 1, WN, T(p.gamma), gfac, 0, d, d_tr);
     __syncwarp();  // the window may be reloaded by the caller's next segment
 
     const double dt = stage_dt(p);
@@ -734,19 +747,19 @@ __global__ void __launch_bounds__(kThreads) stage1d_kernel(StageParams p) {
 // on mbar) instead of per-thread loads. Without TMA, smem holds W and then
 // the y divergences (smem_bytes).
 template <int NDIM, int REC, int LIM, int RS, class T, bool SRC = false, int NT = kThreads, bool TMA = false,
-          bool DEFER = false, bool SCATTER = true>
+          bool DEFER = false, bool SCATTER = true, bool LOW = false>
 __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int bz, T* smem, double& dtmin,
                                        unsigned& flags, const CUtensorMap* tmap = nullptr, uint64_t* mbar = nullptr) {
     constexpr int nh = 2 + NDIM;
     constexpr int NW = NT / 32;
     using G = TileGeom<2, REC>;
-    constexpr int H = G::H, TX = G::TX, TY = G::TY, WX = G::WX, P = G::P, WY = G::WY, PY = G::PY;
+    constexpr int H = G::H, TX = G::TX, TY = G::TY, WX = G::WX, P = G::P, WY = G::WY, PY = G::PY, SX = G::SX;
     constexpr int WV = WY * P;   // per-variable stride of W
     constexpr int YV = TY * PY;  // per-variable stride of dFy
     T* W;
     T* DY;
     if constexpr (TMA) {
-        DY = smem;
+        DY = keeps_stage<NDIM, REC, T>() ? smem + tma_stage_bytes<NDIM, REC>() / sizeof(T) : smem;
         W = reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(smem) + tma_region_bytes<NDIM, REC, T>(p.nvar));
     } else {
         W = smem;
@@ -754,30 +767,49 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
     }
 
     const int x0 = bx * TX;
-    const int y0 = by * TY;
+    // tile height: TY, or at most that (LOW: as a run-time value it costs the
+    // regular kernel 1.5 to 2 %)
+    const int th = LOW ? p.tile_h : TY;
+    const int y0 = by * th;
     const int k = NDIM == 3 ? p.ng + bz : 0;
     const int vw = min(TX, p.nx - x0);
-    const int vh = min(TY, p.ny - y0);
+    const int vh = min(th, p.ny - y0);
+    const bool old = combo_reads_old(p.combo);
+    // TMA: the staged tile; its column xo is the tile's first
+    const double* stg = reinterpret_cast<const double*>(smem);
+    const int xo = SX > WX ? (p.ng - H) & 1 : 0;
+    (void)stg;
+    (void)xo;
 
     // phase 1: primitives of the tile and its cross-shaped halo
-    constexpr int core = TY * WX;
-    constexpr int items = core + 2 * H * TX;
+    const int core = th * WX;
+    const int items = core + 2 * H * TX;
+    if (NDIM == 2 && !DEFER && sizeof(T) == 8 && old) {
+        // the step-start state of the tile's cells, which the finishing reads,
+        // into L2 (one request per 128-byte line): KH 2048^2 stage 0.444 -> 0.436 ms,
+        // MUSCL 0.268 -> 0.260; the FP32 form's is slower with it (0.231 -> 0.236 ms)
+        const long long vs = (long long)p.zc * p.yc * p.xc;
+        for (int it = threadIdx.x; it < vh * 3 * nh; it += NT) {
+            const int v = it / (vh * 3), r = it - v * vh * 3, row = r / 3, l = r - row * 3;
+            const double* a = p.q_old + v * vs + qidx(p, 0, 0, p.ng + y0 + row, p.ng + x0 + min(l * 16, vw - 1));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
+        }
+    }
     bool in_range = p.gas.ok != 0;
     if constexpr (TMA) {
         // the box of WX x WY cells around the tile (x start even: the host
         // only takes this path when ng - H is even), all hydro variables;
         // cells outside the array arrive as zeros and are replaced below
-        double* stg = reinterpret_cast<double*>(smem);
         if (threadIdx.x == 0) {
             mbar_init(mbar, 1);
         }
         __syncthreads();
         if (threadIdx.x == 0) {
-            mbar_expect_tx(mbar, (uint32_t)tma_stage_bytes<NDIM, REC>());
+            mbar_expect_tx(mbar, (uint32_t)(sizeof(double) * nh * SX * (th + 2 * H)));
             if constexpr (NDIM == 3) {
-                tma_load_4d(stg, tmap, p.ng + x0 - H, p.ng + y0 - H, k, 0, mbar);
+                tma_load_4d(smem, tmap, p.ng + x0 - H - xo, p.ng + y0 - H, k, 0, mbar);
             } else {
-                tma_load_3d(stg, tmap, p.ng + x0 - H, p.ng + y0 - H, 0, mbar);
+                tma_load_3d(smem, tmap, p.ng + x0 - H - xo, p.ng + y0 - H, 0, mbar);
             }
         }
         const bool ok = mbar_wait_bounded(mbar, 0, kTmaWaitPolls);
@@ -800,12 +832,12 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
                 const int r = it - core;
                 const int hr = r / TX;
                 tx = r - hr * TX;
-                ty = hr < H ? hr - H : TY + hr - H;
+                ty = hr < H ? hr - H : th + hr - H;
             }
             const int i = p.ng + x0 + tx;
             const int j = p.ng + y0 + ty;
             const bool inb = i >= 0 && i < p.xc && j >= 0 && j < p.yc;
-            flags |= staged_prim<NDIM, T>(p, stg + (ty + H) * WX + (tx + H), WX * WY, inb,
+            flags |= staged_prim<NDIM, T>(p, stg + (ty + H) * SX + (tx + H + xo), SX * (th + 2 * H), inb,
                                           W + (ty + H) * P + (tx + H), WV, in_range);
         }
     } else {
@@ -818,7 +850,7 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
                 const int r = it - core;
                 const int hr = r / TX;
                 tx = r - hr * TX;
-                ty = hr < H ? hr - H : TY + hr - H;
+                ty = hr < H ? hr - H : th + hr - H;
             }
             const int i = p.ng + x0 + tx;
             const int j = p.ng + y0 + ty;
@@ -835,7 +867,6 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
     const int ntr = p.ntracer;
     const double dt = stage_dt(p);
     const double dtdx = dt / p.dx;
-    const bool old = combo_reads_old(p.combo);
     const int c = lane - 1;  // this lane's cell along the sweep
 
     // Two passes through one copy of the sweep code. Pass 0: y faces, one warp
@@ -850,8 +881,9 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
         for (int line = warp; line < nlines; line += NW) {
             const T* centre = axis == 0 ? W + (line + H) * P + (c + H) : W + (c + H) * P + (line + H);
             T d[nh], d_tr[kMaxVars];
-            sweep_line<NDIM, REC, LIM, RS, T>(p, in_range, centre, axis == 0 ? 1 : P, WV, gamma, gfac, axis, d, d_tr);
-            const bool mine = lane >= 1 && lane <= kTile;
+            sweep_line<NDIM, REC, LIM, RS, T>(p, in_range, axis == 0 ? vw : vh, centre, axis == 0 ? 1 : P,
+                                                WV, gamma, gfac, axis, d, d_tr);
+            const bool mine = lane >= 1 && lane <= (axis == 1 ? vh : vw);
             if (axis == 1) {
                 if (mine) {
                     T* dst = DY + c * PY + line;
@@ -865,7 +897,7 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
                 }
                 continue;
             }
-            if (!mine || c >= vw) {
+            if (!mine) {
                 continue;
             }
             const T* dfy = DY + line * PY + c;
@@ -901,7 +933,11 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
                 double qo[nh], qi[nh], qu[nh], sdt[nh];
 #pragma unroll
                 for (int v = 0; v < nh; ++v) {
-                    qi[v] = p.q_in[id0 + v * vs];
+                    if constexpr (TMA && keeps_stage<NDIM, REC, T>()) {
+                        qi[v] = stg[(v * (th + 2 * H) + line + H) * SX + c + H + xo];
+                    } else {
+                        qi[v] = p.q_in[id0 + v * vs];
+                    }
                     qo[v] = old ? p.q_old[id0 + v * vs] : 0.0;
                 }
                 source_dt_of<NDIM, SRC>(p, qi, dt, sdt);
@@ -1009,34 +1045,38 @@ __global__ void __launch_bounds__(kThreads) finish2d_kernel(StageParams p) {
 //   3D FP64 plane pass: five variables' tiles take 90 KB of shared memory,
 //     two CTAs per SM; 384 threads (24 warps at 80 registers) measured 2 %
 //     faster than 320 and 11 % faster than 256.
-template <int NDIM, class T>
+//   LOW (2D grids of at most one tile per SM, see low_tile_rows): one CTA of 512
+//     threads (up to 128 registers) per SM, tiles of p.tile_h rows.
+template <int NDIM, class T, bool LOW = false>
 __host__ __device__ constexpr int tile_threads() {
-    return NDIM == 1 ? kThreads : ((NDIM == 3 && sizeof(T) == 8) ? 384 : 320);
+    return NDIM == 1 ? kThreads : LOW ? 512 : ((NDIM == 3 && sizeof(T) == 8) ? 384 : 320);
 }
-template <int NDIM, class T>
+template <int NDIM, class T, bool LOW = false>
 __host__ __device__ constexpr int tile_min_blocks() {
-    return NDIM == 1 ? (sizeof(T) == 4 ? kMinBlocks2dF32 : kMinBlocks2d) : (sizeof(T) == 4 ? 3 : 2);
+    return LOW ? 1 : NDIM == 1 ? (sizeof(T) == 4 ? kMinBlocks2dF32 : kMinBlocks2d) : (sizeof(T) == 4 ? 3 : 2);
 }
 
 // Whether the TMA tile load fits the kernel's CTAs per SM (shared memory
-// of one SM: 228 KB, 1 KB of it reserved per CTA) and its halo allows an
-// even x start with the usual ng (MUSCL's two-cell halo does not with ng = 3).
+// of one SM: 228 KB, 1 KB of it reserved per CTA). The copy starts at an even x: MUSCL,
+// whose two-cell halo starts at an odd one with ng = 3, stages two columns more and
+// starts one early (2D MUSCL + HLLC stage on 2048^2: 0.287 -> 0.270 ms, FP32 0.32 ->
+// 0.19 ms with what the tile keeps).
 template <int NDIM, int REC, class T>
 __host__ __device__ constexpr bool tma_capable(int nvar) {
-    return REC != kMuscl &&
-           (size_t)tile_min_blocks<NDIM, T>() * (smem_bytes_tma<NDIM, REC, T>(nvar) + 1024 + 256) <= 233472;
+    return (size_t)tile_min_blocks<NDIM, T>() * (smem_bytes_tma<NDIM, REC, T>(nvar) + 1024 + 256) <= 233472;
 }
 
 // DEFER (2D): the tiles write only their x+y divergence into p.dqxy.
-template <int NDIM, int REC, int LIM, int RS, class T, bool SRC = false, bool TMA = false, bool DEFER = false>
-__global__ void __launch_bounds__(tile_threads<NDIM, T>(), tile_min_blocks<NDIM, T>())
+template <int NDIM, int REC, int LIM, int RS, class T, bool SRC = false, bool TMA = false, bool DEFER = false,
+          bool LOW = false>
+__global__ void __launch_bounds__(tile_threads<NDIM, T, LOW>(), tile_min_blocks<NDIM, T, LOW>())
     stage2d_kernel(StageParams p, const __grid_constant__ CUtensorMap tmap) {
     if (p.dt_dev && p.blk->done) {
         return;
     }
     maybe_reset_min(p);
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int NT = tile_threads<NDIM, T>();
+    constexpr int NT = tile_threads<NDIM, T, LOW>();
     __shared__ double red_d[NT / 32];
     __shared__ unsigned red_u[NT / 32];
     __shared__ __align__(8) uint64_t mbar;
@@ -1057,11 +1097,12 @@ __global__ void __launch_bounds__(tile_threads<NDIM, T>(), tile_min_blocks<NDIM,
     // stores, and the FP64 FOG, MUSCL and PPM kernels with HLLC went from
     // none to about 490.
     constexpr bool kAfter = NDIM == 2 && !DEFER && sizeof(T) == 8 && REC == kWeno5z;
-    tile2d<NDIM, REC, LIM, RS, T, SRC, NT, TMA, DEFER, !kAfter>(p, blockIdx.x, by, blockIdx.z,
-                                                                reinterpret_cast<T*>(base), dtmin, flags, &tmap, &mbar);
+    tile2d<NDIM, REC, LIM, RS, T, SRC, NT, TMA, DEFER, !kAfter, LOW>(
+        p, blockIdx.x, by, blockIdx.z, reinterpret_cast<T*>(base), dtmin, flags, &tmap, &mbar);
     if constexpr (kAfter) {
-        const int x0 = blockIdx.x * kTile, y0 = by * kTile;
-        const int vw = min(kTile, p.nx - x0), vh = min(kTile, p.ny - y0);
+        const int th = LOW ? p.tile_h : kTile;
+        const int x0 = blockIdx.x * kTile, y0 = by * th;
+        const int vw = min(kTile, p.nx - x0), vh = min(th, p.ny - y0);
         if (x0 < p.ng || x0 + vw > p.nx - p.ng || y0 < p.ng || y0 + vh > p.ny - p.ng) {
             __syncthreads();
             const long long vs = (long long)p.zc * p.yc * p.xc;
@@ -1236,7 +1277,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks2d)
     for (int col = warp; col < vw; col += kWarps) {
         T* centre = W + (c + H) * PZ + col;
         T d[nh], d_tr[kMaxVars];
-        sweep_line<NDIM, REC, LIM, RS, T>(p, in_range, centre, PZ, WV, gamma, gfac, 2, d, d_tr);
+        sweep_line<NDIM, REC, LIM, RS, T>(p, in_range, vh, centre, PZ, WV, gamma, gfac, 2, d, d_tr);
         __syncwarp();
         if (lane >= 1 && lane <= TZ) {
 #pragma unroll
