@@ -560,6 +560,32 @@ mc_status step_host_pipelined(mc_ctx* c, double* Qh, double* Q, const mc_clock* 
     return MC_OK;
 }
 
+// Whether the device-driven loop takes its steps in the one-launch form of small
+// 1D problems (run1d_impl.cuh): no work between the stages but the stage kernel's own.
+// us per step, separate launches -> one launch (FP64): MUSCL + HLLC, rk2, 64 cells 20.5 ->
+// 6.9, 1024 17.4 -> 7.3, 3840 17.8 -> 9.2, 7680 21.5 -> 15.4; WENO5-Z + HLLC, ssprk3, 1024
+// 29.7 -> 11.7, 3840 27.6 -> 16.7, 7680 30.1 -> 30.0; beyond 256 segments (7680 cells) eight
+// SMs take longer than the launches.
+bool runs_whole_steps(const mc_ctx* c) {
+    return c->grid.num_dim == 1 && c->eos_type == mc::kEosIdeal && !c->user_bc && !c->slab && !c->cfl_hook &&
+           !c->profiling && (c->nx + mc::kTile - 1) / mc::kTile <= mc::kRun1dMaxSegments;
+}
+
+mc_status enqueue_run1d(mc_ctx* c, double* Q, int64_t steps, double* dt_log, cudaStream_t s) {
+    const mc::StagePlan plan = mc::plan_for(c->scheme.time_stepper);
+    double* bufs[3] = {Q, c->buf_a, c->buf_b};
+    double* last_in = bufs[plan.in[plan.n - 1]];
+    c->last_stage_in = last_in;
+    const StageParams p = base_params(c);
+    const int r = c->scheme.reconstruction, l = c->scheme.slope_limiter, rs = c->scheme.riemann_solver;
+    c->launches += 1;
+    MC_CUDA(c->scheme.precision == MC_PRECISION_FP32_COMPENSATED
+                ? mc::launch_run1d_fp32(p, r, l, rs, Q, last_in, plan, steps, dt_log, s)
+                : mc::launch_run1d_fp64(p, r, l, rs, Q, last_in, plan, steps, dt_log, s),
+            "1D run");
+    return MC_OK;
+}
+
 // The domain-wide reduction of the CFL minimum word: the slab
 // decomposition's all-reduce and the caller's hook, if any.
 mc_status reduce_cfl(mc_ctx* c, cudaStream_t s) {
@@ -1083,11 +1109,17 @@ mc_status mc_advance(mc_ctx* c, double* Q, mc_clock* clock, int64_t max_steps, i
     MC_CUDA(mc::launch_clock_advance(c->blk, dlog, 1, s), "clock");
     c->launches += 4;
     const double* dt_dev = &c->blk->dt;
-    const int64_t chunk = 64;
+    const bool whole = runs_whole_steps(c);
+    const int64_t chunk = whole ? 1024 : 64;
     int64_t issued = 0;
     while (issued < max_steps) {
         const int64_t n = std::min(chunk, max_steps - issued);
-        for (int64_t k = 0; k < n; ++k) {
+        if (whole) {
+            if (mc_status st = enqueue_run1d(c, Q, n, dlog, s)) {
+                return st;
+            }
+        }
+        for (int64_t k = 0; !whole && k < n; ++k) {
             if (mc_status st = enqueue_step(c, Q, 0.0, dt_dev, false, s)) {
                 return st;
             }

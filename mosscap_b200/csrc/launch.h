@@ -51,6 +51,17 @@ cudaError_t launch_stage_d2_fp32_defer(const StageParams& p, int rec, int lim, i
 cudaError_t launch_stage_d2_fp64_src_defer(const StageParams& p, int rec, int lim, int rs, int pass, cudaStream_t s);
 cudaError_t launch_stage_d2_fp32_src_defer(const StageParams& p, int rec, int lim, int rs, int pass, cudaStream_t s);
 
+// Up to `steps` whole steps of a small 1D problem's device-driven loop in one
+// launch (run1d_impl.cuh): Q, the buffer that receives the last stage's input, the
+// clock in p.blk (its dt set), the dt log (or null). For problems of at most
+// kRun1dMaxSegments 30-cell segments.
+constexpr int kRun1dCtas = 8, kRun1dWarps = 16;
+constexpr int kRun1dMaxSegments = 2 * kRun1dCtas * kRun1dWarps;
+cudaError_t launch_run1d_fp64(const StageParams& p, int rec, int lim, int rs, double* Q, double* last_in,
+                              const StagePlan& plan, long long steps, double* dt_log, cudaStream_t s);
+cudaError_t launch_run1d_fp32(const StageParams& p, int rec, int lim, int rs, double* Q, double* last_in,
+                              const StagePlan& plan, long long steps, double* dt_log, cudaStream_t s);
+
 // Ghost fill of Q from its interior (every built-in boundary kind).
 cudaError_t launch_fill_bcs(const StageParams& p, int ndim, cudaStream_t s);
 // Primitives of p.q_in over every cell (ghosts included) into w, tracers
