@@ -81,14 +81,13 @@ __host__ __device__ constexpr size_t tma_stage_bytes() {
     using G = TileGeom<2, REC>;
     return sizeof(double) * (size_t)(2 + NDIM) * G::WY * G::SX;
 }
-// Whether the staged tile outlives the conversion (2D, FP64; FP32 MUSCL and FOG):
-// the y divergences then lie after it, and the finishing takes each
-// cell's stage input from it.
-// Shared memory still allows two CTAs per SM (FP32 three). Measured with the stage input
+// Whether the staged tile outlives the conversion (2D, FP64): the y divergences
+// then lie after it, and the finishing takes each cell's stage input from it.
+// Shared memory still allows two CTAs per SM. Measured with the stage input
 // from L2 -> from the staged tile: KH 2048^2 stage 0.451 -> 0.444 ms, PPM + HLL 0.336 -> 0.332.
 template <int NDIM, int REC, class T>
 __host__ __device__ constexpr bool keeps_stage() {
-    return NDIM == 2 && (sizeof(T) == 8 || halo_of<REC>() < 3);
+    return NDIM == 2 && sizeof(T) == 8;
 }
 template <int NDIM, int REC, class T>
 __host__ __device__ constexpr size_t tma_region_bytes(int nvar) {
@@ -324,14 +323,11 @@ __device__ __forceinline__ bool prim_for_sweep(double gamma, const FastGas& gas,
     }
 }
 
-// Load one cell's conserved variables from q_in and store its primitives
-// (tracers divided by rho, source/Hydro.cpp:27-33) into shared memory.
-// Clears in_range unless the cell is in range for the FP64 sweep.
-template <int NDIM, class T>
-__device__ __forceinline__ unsigned load_prim(const StageParams& p, int k, int j, int i, bool inb, T* w_smem,
-                                              int var_stride, bool& in_range) {
+// One cell's conserved variables from q_in, or, outside the array, a benign
+// state that no stored result depends on.
+template <int NDIM>
+__device__ __forceinline__ void load_cons(const StageParams& p, int k, int j, int i, bool inb, double* q) {
     constexpr int nh = 2 + NDIM;
-    double q[nh], w[nh];
     const long long vs = (long long)p.zc * p.yc * p.xc;  // variable stride of the state
     const long long id0 = qidx(p, 0, k, j, i);
     if (inb) {
@@ -340,7 +336,6 @@ __device__ __forceinline__ unsigned load_prim(const StageParams& p, int k, int j
             q[v] = p.q_in[id0 + v * vs];
         }
     } else {
-        // outside the array: a benign state that no stored result depends on
         q[0] = 1.0;
 #pragma unroll
         for (int v = 1; v < nh - 1; ++v) {
@@ -348,6 +343,16 @@ __device__ __forceinline__ unsigned load_prim(const StageParams& p, int k, int j
         }
         q[nh - 1] = 1.0;
     }
+}
+
+// Store the primitives of the cell whose conserved variables load_cons read
+// (tracers, loaded here, divided by rho, source/Hydro.cpp:27-33) into shared memory.
+// Clears in_range unless the cell is in range for the FP64 sweep.
+template <int NDIM, class T>
+__device__ __forceinline__ unsigned store_prim(const StageParams& p, int k, int j, int i, bool inb, const double* q,
+                                               T* w_smem, int var_stride, bool& in_range) {
+    constexpr int nh = 2 + NDIM;
+    double w[nh];
     const bool ok = prim_for_sweep<NDIM, T>(p.gamma, p.gas, q, w);
     in_range = in_range && ok;
 #pragma unroll
@@ -355,6 +360,8 @@ __device__ __forceinline__ unsigned load_prim(const StageParams& p, int k, int j
         w_smem[v * var_stride] = T(w[v]);
     }
     if (p.ntracer > 0) {
+        const long long vs = (long long)p.zc * p.yc * p.xc;
+        const long long id0 = qidx(p, 0, k, j, i);
         const double inv_rho = 1.0 / q[0];
         for (int t = 0; t < p.ntracer; ++t) {
             const double qt = inb ? p.q_in[id0 + (nh + t) * vs] : 0.0;
@@ -374,6 +381,14 @@ __device__ __forceinline__ unsigned load_prim(const StageParams& p, int k, int j
         fin = fin && isfinite(q[v]);
     }
     return state_flags(w[0], w[nh - 1], fin);
+}
+
+template <int NDIM, class T>
+__device__ __forceinline__ unsigned load_prim(const StageParams& p, int k, int j, int i, bool inb, T* w_smem,
+                                              int var_stride, bool& in_range) {
+    double q[2 + NDIM];
+    load_cons<NDIM>(p, k, j, i, inb, q);
+    return store_prim<NDIM, T>(p, k, j, i, inb, q, w_smem, var_stride, in_range);
 }
 
 // The same as load_prim for a cell whose conserved variables sit in the
@@ -841,21 +856,52 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
                                           W + (ty + H) * P + (tx + H), WV, in_range);
         }
     } else {
-        for (int it = threadIdx.x; it < items; it += NT) {
-            int tx, ty;
-            if (it < core) {
-                ty = it / WX;
-                tx = it - ty * WX - H;
-            } else {
-                const int r = it - core;
-                const int hr = r / TX;
-                tx = r - hr * TX;
-                ty = hr < H ? hr - H : th + hr - H;
+        // UL cells of a thread at a time, their loads issued together (one at a time ->
+        // four, stage on 2048^2: FP64 MUSCL + HLLC 0.274 -> 0.262 ms, PPM + HLL 0.344 ->
+        // 0.336; FP32 MUSCL 0.184 -> 0.176; Sedov 256^3 FP32 plane pass 0.772 -> 0.746)
+        constexpr int UL = 4;
+#pragma unroll 1
+        for (int base = threadIdx.x; base < items; base += UL * NT) {
+            double q[UL][nh];
+#pragma unroll
+            for (int u = 0; u < UL; ++u) {
+                const int it = base + u * NT;
+                int tx, ty;
+                if (it < core) {
+                    ty = it / WX;
+                    tx = it - ty * WX - H;
+                } else {
+                    const int r = it - core;
+                    const int hr = r / TX;
+                    tx = r - hr * TX;
+                    ty = hr < H ? hr - H : th + hr - H;
+                }
+                const int i = p.ng + x0 + tx;
+                const int j = p.ng + y0 + ty;
+                const bool inb = it < items && i >= 0 && i < p.xc && j >= 0 && j < p.yc;
+                load_cons<NDIM>(p, k, j, i, inb, q[u]);
             }
-            const int i = p.ng + x0 + tx;
-            const int j = p.ng + y0 + ty;
-            const bool inb = i >= 0 && i < p.xc && j >= 0 && j < p.yc;
-            flags |= load_prim<NDIM, T>(p, k, j, i, inb, W + (ty + H) * P + (tx + H), WV, in_range);
+#pragma unroll
+            for (int u = 0; u < UL; ++u) {
+                const int it = base + u * NT;
+                if (it >= items) {
+                    break;
+                }
+                int tx, ty;
+                if (it < core) {
+                    ty = it / WX;
+                    tx = it - ty * WX - H;
+                } else {
+                    const int r = it - core;
+                    const int hr = r / TX;
+                    tx = r - hr * TX;
+                    ty = hr < H ? hr - H : th + hr - H;
+                }
+                const int i = p.ng + x0 + tx;
+                const int j = p.ng + y0 + ty;
+                const bool inb = i >= 0 && i < p.xc && j >= 0 && j < p.yc;
+                flags |= store_prim<NDIM, T>(p, k, j, i, inb, q[u], W + (ty + H) * P + (tx + H), WV, in_range);
+            }
         }
     }
     in_range = __syncthreads_and(in_range);
@@ -1059,11 +1105,12 @@ __host__ __device__ constexpr int tile_min_blocks() {
 // Whether the TMA tile load fits the kernel's CTAs per SM (shared memory
 // of one SM: 228 KB, 1 KB of it reserved per CTA). The copy starts at an even x: MUSCL,
 // whose two-cell halo starts at an odd one with ng = 3, stages two columns more and
-// starts one early (2D MUSCL + HLLC stage on 2048^2: 0.287 -> 0.270 ms, FP32 0.32 ->
-// 0.19 ms with what the tile keeps).
+// starts one early. FP32 MUSCL loads per thread (stage on 2048^2 0.176 ms, 0.188 with
+// the copy; FP64 MUSCL is the same either way, WENO5-Z and PPM gain 2 to 5 %).
 template <int NDIM, int REC, class T>
 __host__ __device__ constexpr bool tma_capable(int nvar) {
-    return (size_t)tile_min_blocks<NDIM, T>() * (smem_bytes_tma<NDIM, REC, T>(nvar) + 1024 + 256) <= 233472;
+    return !(REC == kMuscl && sizeof(T) == 4) &&
+           (size_t)tile_min_blocks<NDIM, T>() * (smem_bytes_tma<NDIM, REC, T>(nvar) + 1024 + 256) <= 233472;
 }
 
 // DEFER (2D): the tiles write only their x+y divergence into p.dqxy.
