@@ -30,9 +30,11 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "adjoint_physics.cuh"
+#include "blocks.h"
 #include "launch.h"
 #include "mosscap_b200.h"
 #include "slab.h"
@@ -408,6 +410,8 @@ __global__ void zero_kernel(double* p, long long n) {
 } // namespace
 
 struct mc_adjoint {
+    int device = 0;
+    std::vector<std::pair<void*, size_t>> blocks;  // its device memory (blocks.h)
     mc_grid grid{};
     mc_scheme scheme{};
     int k = 20;                 // checkpoint interval
@@ -460,6 +464,35 @@ mc_status afail(mc_status s, const std::string& msg) {
             return afail(MC_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e_)); \
         }                                                                                  \
     } while (0)
+
+// A block of device memory that belongs to the adjoint until free_block or
+// its end.
+template <class T>
+cudaError_t alloc_block(mc_adjoint* a, T** p, size_t bytes) {
+    const cudaError_t e = mc::block_alloc((void**)p, bytes);
+    if (e == cudaSuccess) {
+        a->blocks.emplace_back((void*)*p, bytes);
+    }
+    return e;
+}
+
+// Give blocks back; work that uses them may still be pending.
+void free_blocks(mc_adjoint* a, std::initializer_list<void*> ps) {
+    const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+    for (void* p : ps) {
+        for (size_t k = 0; p && k < a->blocks.size(); ++k) {
+            if (a->blocks[k].first == p) {
+                if (idle) {
+                    mc::block_free(p, a->blocks[k].second, a->device);
+                } else {
+                    cudaFree(p);
+                }
+                a->blocks.erase(a->blocks.begin() + k);
+                break;
+            }
+        }
+    }
+}
 
 StageParams fwd_params(const mc_adjoint* a) {
     StageParams p;
@@ -596,27 +629,28 @@ mc_status grow(mc_adjoint* a, int64_t steps) {
     // the segment buffer: (3 k + 1) states for segments of k = min(interval, steps) steps
     const int64_t k_eff = steps < a->k ? (steps > 0 ? steps : 1) : a->k;
     if (k_eff > a->seg_cap) {
-        cudaFree(a->seg);
+        if (a->seg) {
+            free_blocks(a, {a->seg});
+        }
         a->seg = nullptr;
         a->seg_cap = 0;
-        MCA_CUDA(cudaMalloc(&a->seg, sizeof(double) * a->state * (3 * (size_t)k_eff + 1)), "alloc segment");
+        MCA_CUDA(alloc_block(a, &a->seg, sizeof(double) * a->state * (3 * (size_t)k_eff + 1)), "alloc segment");
         a->seg_cap = k_eff;
     }
     // the records hold steps + 1 entries (a run of 0 steps still records its first dt)
     if (a->dts && a->mins && a->clamped && a->ckpt && steps <= a->rec_cap) {
         return MC_OK;
     }
-    cudaFree(a->dts);
-    cudaFree(a->mins);
-    cudaFree(a->clamped);
-    cudaFree(a->ckpt);
+    if (a->dts || a->mins || a->clamped || a->ckpt) {
+        free_blocks(a, {a->dts, a->mins, a->clamped, a->ckpt});
+    }
     a->dts = a->mins = a->ckpt = nullptr;
     a->clamped = nullptr;
     const int64_t nck = steps / a->k + 1;
-    MCA_CUDA(cudaMalloc(&a->dts, sizeof(double) * (steps + 1)), "alloc");
-    MCA_CUDA(cudaMalloc(&a->mins, sizeof(double) * (steps + 1)), "alloc");
-    MCA_CUDA(cudaMalloc(&a->clamped, sizeof(int) * (steps + 1)), "alloc");
-    MCA_CUDA(cudaMalloc(&a->ckpt, sizeof(double) * a->state * nck), "alloc checkpoints");
+    MCA_CUDA(alloc_block(a, &a->dts, sizeof(double) * (steps + 1)), "alloc");
+    MCA_CUDA(alloc_block(a, &a->mins, sizeof(double) * (steps + 1)), "alloc");
+    MCA_CUDA(alloc_block(a, &a->clamped, sizeof(int) * (steps + 1)), "alloc");
+    MCA_CUDA(alloc_block(a, &a->ckpt, sizeof(double) * a->state * nck), "alloc checkpoints");
     a->rec_cap = steps;
     return MC_OK;
 }
@@ -679,10 +713,10 @@ mc_status slab_prepare(mc_adjoint* a, int32_t rank, int32_t world) {
     // one block holds the VJP halos ([4][kAH][xc] + [4][kMH][xc]) or ng ghost rows
     a->halo_cap = 4LL * (kAH + kMH > a->grid.ng ? kAH + kMH : a->grid.ng) * a->grid.xc;
     if (!a->send) {
-        MCA_CUDA(cudaMalloc(&a->send, sizeof(double) * 2 * (size_t)a->halo_cap), "alloc halo");
+        MCA_CUDA(alloc_block(a, &a->send, sizeof(double) * 2 * (size_t)a->halo_cap), "alloc halo");
     }
     if (!a->recv) {
-        MCA_CUDA(cudaMalloc(&a->recv, sizeof(double) * 2 * (size_t)a->halo_cap), "alloc halo");
+        MCA_CUDA(alloc_block(a, &a->recv, sizeof(double) * 2 * (size_t)a->halo_cap), "alloc halo");
     }
     return MC_OK;
 }
@@ -716,6 +750,7 @@ mc_status mc_adjoint_create(const mc_grid* grid, const mc_scheme* scheme, int32_
     if (!a) {
         return afail(MC_ERR_OUT_OF_MEMORY, "host allocation");
     }
+    cudaGetDevice(&a->device);
     a->grid = g;
     a->scheme = s;
     a->k = checkpoint_every;
@@ -727,7 +762,7 @@ mc_status mc_adjoint_create(const mc_grid* grid, const mc_scheme* scheme, int32_
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void** p, size_t bytes) {
         if (e == cudaSuccess) {
-            e = cudaMalloc(p, bytes);
+            e = alloc_block(a, p, bytes);
         }
     };
     const size_t sb = sizeof(double) * a->state;
@@ -762,25 +797,19 @@ mc_status mc_adjoint_destroy(mc_adjoint* a) {
     if (!a) {
         return MC_OK;
     }
-    cudaFree(a->ckpt);
-    cudaFree(a->seg);
-    cudaFree(a->work_a);
-    cudaFree(a->work_b);
-    for (auto l : a->lam) {
-        cudaFree(l);
+    // the blocks may be handed to another adjoint: nothing may still use them
+    int device = a->device;
+    cudaGetDevice(&device);
+    cudaSetDevice(a->device);
+    const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+    for (const auto& b : a->blocks) {
+        if (idle) {
+            mc::block_free(b.first, b.second, a->device);
+        } else {
+            cudaFree(b.first);
+        }
     }
-    cudaFree(a->acc);
-    cudaFree(a->dts);
-    cudaFree(a->mins);
-    cudaFree(a->clamped);
-    cudaFree(a->blk);
-    cudaFree(a->blk_rec);
-    cudaFree(a->part);
-    cudaFree(a->scal);
-    cudaFree(a->argmin);
-    cudaFree(a->key);
-    cudaFree(a->send);
-    cudaFree(a->recv);
+    cudaSetDevice(device);
     mc::slab_destroy(a->slab);
     delete a;
     return MC_OK;
