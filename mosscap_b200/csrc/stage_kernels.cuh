@@ -859,7 +859,9 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
         // UL cells of a thread at a time, their loads issued together (one at a time ->
         // four, stage on 2048^2: FP64 MUSCL + HLLC 0.274 -> 0.262 ms, PPM + HLL 0.344 ->
         // 0.336; FP32 MUSCL 0.184 -> 0.176; Sedov 256^3 FP32 plane pass 0.772 -> 0.746)
-        constexpr int UL = 4;
+        // (the batched kernel, SCATTER false, spills with four: 384 problems, 4 steps, FP64 8.93,
+        // 8.43, 8.99 ms with one, two, four; FP32 6.62 and 6.32 with one and two)
+        constexpr int UL = SCATTER ? 4 : 2;
 #pragma unroll 1
         for (int base = threadIdx.x; base < items; base += UL * NT) {
             double q[UL][nh];
