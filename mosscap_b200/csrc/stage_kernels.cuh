@@ -448,12 +448,11 @@ __host__ __device__ constexpr int recon_group() {
 // neighbouring cells along the axis in shared memory, `vstride` between
 // variables. The axis is a runtime value so that both directions run the
 // same instructions.
-template <int NDIM, int REC, int LIM, int RS, class T>
+template <int NDIM, int REC, int LIM, int RS, class T, int G = recon_group<NDIM, REC>()>
 __device__ __forceinline__ void face_sweep(const T* centre, int stride, int vstride, int ntracer, T gamma, T gfac,
                                            int axis, T* d, T* d_tr) {
     constexpr int nh = 2 + NDIM;
     constexpr int S = stencil_half<REC>();
-    constexpr int G = recon_group<NDIM, REC>();
     T wl[nh], wr[nh];
     if constexpr (G < nh) {
         // a rolled loop over groups of G variables (a smaller instruction
@@ -527,13 +526,15 @@ __device__ __forceinline__ void face_sweep(const T* centre, int stride, int vstr
 }
 
 // face_sweep on double in a call of its own: d into out[0..nh), the tracers'
-// d_tr after it. The FP64 sweep's form for values out of range.
-template <int NDIM, int REC, int LIM, int RS>
+// d_tr after it. The FP64 sweep's form for values out of range. G: variables per
+// iteration of its loop; what it needs shows in its callers' registers (see
+// ztile3d_kernel).
+template <int NDIM, int REC, int LIM, int RS, int G>
 __device__ __noinline__ void face_sweep_any(const double* centre, int stride, int vstride, int ntracer, double gamma,
                                             double gfac, int axis, double* out) {
     constexpr int nh = 2 + NDIM;
     double d[nh], d_tr[kMaxVars];
-    face_sweep<NDIM, REC, LIM, RS, double>(centre, stride, vstride, ntracer, gamma, gfac, axis, d, d_tr);
+    face_sweep<NDIM, REC, LIM, RS, double, G>(centre, stride, vstride, ntracer, gamma, gfac, axis, d, d_tr);
 #pragma unroll
     for (int v = 0; v < nh; ++v) {
         out[v] = d[v];
@@ -626,7 +627,7 @@ __device__ __forceinline__ bool fast_face_sweep(const double* centre, int stride
 // (warp-uniform): every value the line's stencils read is in range; cells: the
 // number of cells from lane 1 on whose divergence is wanted; a line
 // that is not, or whose face states are not, takes face_sweep's own code.
-template <int NDIM, int REC, int LIM, int RS, class T>
+template <int NDIM, int REC, int LIM, int RS, class T, int GA = recon_group<NDIM, REC>()>
 __device__ __forceinline__ void sweep_line(const StageParams& p, bool in_range, int cells, const T* centre,
                                            int stride, int vstride, T gamma, T gfac, int axis, T* d, T* d_tr) {
     if constexpr (sizeof(T) == 8) {
@@ -640,7 +641,7 @@ __device__ __forceinline__ void sweep_line(const StageParams& p, bool in_range, 
         const int lane = threadIdx.x & 31;
         if (__any_sync(0xffffffffu, redo && lane >= 1 && lane <= cells + 1)) {
             double out[kMaxVars];
-            face_sweep_any<NDIM, REC, LIM, RS>(centre, stride, vstride, p.ntracer, gamma, gfac, axis, out);
+            face_sweep_any<NDIM, REC, LIM, RS, GA>(centre, stride, vstride, p.ntracer, gamma, gfac, axis, out);
 #pragma unroll
             for (int v = 0; v < nh; ++v) {
                 d[v] = out[v];
@@ -1321,12 +1322,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks2d)
     const int c = lane - 1;  // this lane's cell along the column
 
     // phase 2: z sweeps, one warp per column; the divergence replaces the
-    // column's primitives once every lane has read its stencil
+    // column's primitives once every lane has read its stencil. The out-of-range
+    // form one variable per iteration: Sedov 256^3 FP64 z pass 1.18 -> 1.14 ms (the
+    // plane pass is slower with it, 1.33 -> 1.35)
 #pragma unroll 1
     for (int col = warp; col < vw; col += kWarps) {
         T* centre = W + (c + H) * PZ + col;
         T d[nh], d_tr[kMaxVars];
-        sweep_line<NDIM, REC, LIM, RS, T>(p, in_range, vh, centre, PZ, WV, gamma, gfac, 2, d, d_tr);
+        sweep_line<NDIM, REC, LIM, RS, T, 1>(p, in_range, vh, centre, PZ, WV, gamma, gfac, 2, d, d_tr);
         __syncwarp();
         if (lane >= 1 && lane <= TZ) {
 #pragma unroll

@@ -54,16 +54,12 @@ __global__ void __launch_bounds__(256) cfl_min_kernel(StageParams p) {
     unsigned flags = 0;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < p.plane;
          c += (long long)gridDim.x * blockDim.x) {
-        double q[nh], w[nh];
-        bool fin = true;
+        double q[nh];
 #pragma unroll
         for (int v = 0; v < nh; ++v) {
             q[v] = p.q_in[v * p.plane + c];
-            fin = fin && isfinite(q[v]);
         }
-        prim_from_cons<NDIM>(p.gamma, q, w);
-        flags |= state_flags(w[0], w[nh - 1], fin);
-        m = smin(cfl_dt<NDIM>(p.gamma, p.dx, w), m);
+        m = smin(cfl_bound_of<NDIM, double>(p, q, &flags), m);
     }
     block_publish(m, flags, true, p.blk, red_d, red_u);
 }
