@@ -774,9 +774,6 @@ mc_status mc_adjoint_create(const mc_grid* grid, const mc_scheme* scheme, int32_
     alloc((void**)&a->acc, sb);
     alloc((void**)&a->blk, sizeof(DeviceBlock));
     alloc((void**)&a->blk_rec, sizeof(DeviceBlock));
-    if (e == cudaSuccess) {
-        e = cudaMemset(a->blk_rec, 0, sizeof(DeviceBlock));
-    }
     alloc((void**)&a->part, sizeof(double) * 2 * a->tiles);
     alloc((void**)&a->scal, sizeof(double) * 2);
     alloc((void**)&a->argmin, sizeof(int));
@@ -871,6 +868,9 @@ mc_status mc_adjoint_backward(mc_adjoint* a, double* lambda, double* dgamma, voi
     }
     const cudaStream_t s = (cudaStream_t)stream;
     const size_t sb = sizeof(double) * a->state;
+    // in the caller's stream: a memset elsewhere is not ordered before the recompute
+    // stages, and a stale `done` would make them return at once
+    MCA_CUDA(cudaMemsetAsync(a->blk_rec, 0, sizeof(DeviceBlock), s), "recompute clock");
     zero_kernel<<<64, 256, 0, s>>>(a->scal, 2);
     MCA_CUDA(cudaMemcpyAsync(a->lam[0], lambda, sb, cudaMemcpyDeviceToDevice, s), "lambda in");
     double* L3 = a->lam[0];
