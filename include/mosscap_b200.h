@@ -379,6 +379,23 @@ typedef struct mc_adjoint mc_adjoint;
 
 mc_status mc_adjoint_create(const mc_grid* grid, const mc_scheme* scheme, int32_t checkpoint_every,
                             mc_adjoint** out);
+/* The same with the caller's device memory (memory NULL: cudaMalloc and
+ * cudaFree), for callers that make and drop adjoints often: allocating and
+ * freeing device memory waits for the device and takes milliseconds.
+ * alloc(user, bytes) returns memory of the device current at this call,
+ * aligned to 256 bytes, or NULL when there is none (the call that needs it
+ * fails as when cudaMalloc does); its contents are arbitrary, and work of the
+ * caller still pending on it must be ordered before what the adjoint enqueues
+ * in the stream of mc_adjoint_forward. The adjoint calls it here, in mc_adjoint_forward and in
+ * mc_adjoint_set_slab_*, and free(user, p) there and in mc_adjoint_destroy,
+ * after the device has finished all work. *memory is copied. */
+typedef struct mc_allocator {
+    void* (*alloc)(void* user, uint64_t bytes);
+    void (*free)(void* user, void* p);
+    void* user;
+} mc_allocator;
+mc_status mc_adjoint_create_in(const mc_grid* grid, const mc_scheme* scheme, int32_t checkpoint_every,
+                               const mc_allocator* memory, mc_adjoint** out);
 mc_status mc_adjoint_destroy(mc_adjoint* adj);
 /* Advance Q (ghosts filled) by exactly n_steps steps in place, each with
  * dt = compute_dt under *clock (which must not reach max_time within the run),

@@ -83,6 +83,15 @@ COMM_FN = ctypes.CFUNCTYPE(ctypes.c_int32, ctypes.c_void_p, ctypes.c_int32, ctyp
 COMM_HALO, COMM_MIN_U64, COMM_SUM_F64, COMM_MIN_I64 = 0, 1, 2, 3
 
 
+# device memory from the caller: alloc(user, bytes) -> address or None, free(user, address)
+ALLOC_FN = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64)
+FREE_FN = ctypes.CFUNCTYPE(None, ctypes.c_void_p, ctypes.c_void_p)
+
+
+class McAllocator(ctypes.Structure):
+    _fields_ = [("alloc", ALLOC_FN), ("free", FREE_FN), ("user", ctypes.c_void_p)]
+
+
 class McEosTable(ctypes.Structure):
     _fields_ = [
         ("log_eint_rho_start", ctypes.c_double), ("log_eint_rho_step", ctypes.c_double),
@@ -183,6 +192,8 @@ def load() -> ctypes.CDLL:
     lib.mc_launch_count.restype = i64
     lib.mc_adjoint_create.argtypes = [P(McGrid), P(McScheme), i32, P(vp)]
     lib.mc_adjoint_create.restype = i32
+    lib.mc_adjoint_create_in.argtypes = [P(McGrid), P(McScheme), i32, P(McAllocator), P(vp)]
+    lib.mc_adjoint_create_in.restype = i32
     lib.mc_adjoint_destroy.argtypes = [vp]
     lib.mc_adjoint_destroy.restype = i32
     lib.mc_adjoint_forward.argtypes = [vp, vp, P(McClock), i64, vp]

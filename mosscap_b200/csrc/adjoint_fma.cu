@@ -28,13 +28,12 @@
 
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <new>
 #include <string>
-#include <utility>
 #include <vector>
 
 #include "adjoint_physics.cuh"
-#include "blocks.h"
 #include "launch.h"
 #include "mosscap_b200.h"
 #include "slab.h"
@@ -411,7 +410,8 @@ __global__ void zero_kernel(double* p, long long n) {
 
 struct mc_adjoint {
     int device = 0;
-    std::vector<std::pair<void*, size_t>> blocks;  // its device memory (blocks.h)
+    mc_allocator memory{};       // alloc null: cudaMalloc and cudaFree
+    void* blocks[24] = {};       // its device memory (19 blocks at most)
     mc_grid grid{};
     mc_scheme scheme{};
     int k = 20;                 // checkpoint interval
@@ -465,32 +465,49 @@ mc_status afail(mc_status s, const std::string& msg) {
         }                                                                                  \
     } while (0)
 
-// A block of device memory that belongs to the adjoint until free_block or
-// its end.
+// A block of device memory that belongs to the adjoint until free_blocks.
 template <class T>
 cudaError_t alloc_block(mc_adjoint* a, T** p, size_t bytes) {
-    const cudaError_t e = mc::block_alloc((void**)p, bytes);
-    if (e == cudaSuccess) {
-        a->blocks.emplace_back((void*)*p, bytes);
+    void** slot = a->blocks;
+    while (*slot) {
+        ++slot;
     }
-    return e;
+    if (a->memory.alloc) {
+        *slot = a->memory.alloc(a->memory.user, bytes);
+        if (!*slot) {
+            return cudaErrorMemoryAllocation;
+        }
+    } else if (const cudaError_t e = cudaMalloc(slot, bytes)) {
+        *slot = nullptr;
+        return e;
+    }
+    *p = (T*)*slot;
+    return cudaSuccess;
 }
 
-// Give blocks back; work that uses them may still be pending.
-void free_blocks(mc_adjoint* a, std::initializer_list<void*> ps) {
-    const bool idle = cudaDeviceSynchronize() == cudaSuccess;
-    for (void* p : ps) {
-        for (size_t k = 0; p && k < a->blocks.size(); ++k) {
-            if (a->blocks[k].first == p) {
-                if (idle) {
-                    mc::block_free(p, a->blocks[k].second, a->device);
-                } else {
-                    cudaFree(p);
-                }
-                a->blocks.erase(a->blocks.begin() + k);
-                break;
-            }
+// Give the blocks among ps (or all) back once no work uses them (cudaFree waits by itself).
+void free_blocks(mc_adjoint* a, std::initializer_list<void*> ps, bool all = false) {
+    if (a->memory.alloc) {
+        int device = a->device;
+        cudaGetDevice(&device);
+        cudaSetDevice(a->device);
+        cudaDeviceSynchronize();
+        cudaSetDevice(device);
+    }
+    for (void*& b : a->blocks) {
+        bool wanted = all;
+        for (void* p : ps) {
+            wanted = wanted || p == b;
         }
+        if (!b || !wanted) {
+            continue;
+        }
+        if (a->memory.alloc) {
+            a->memory.free(a->memory.user, b);
+        } else {
+            cudaFree(b);
+        }
+        b = nullptr;
     }
 }
 
@@ -727,10 +744,18 @@ extern "C" {
 
 mc_status mc_adjoint_create(const mc_grid* grid, const mc_scheme* scheme, int32_t checkpoint_every,
                             mc_adjoint** out) {
+    return mc_adjoint_create_in(grid, scheme, checkpoint_every, nullptr, out);
+}
+
+mc_status mc_adjoint_create_in(const mc_grid* grid, const mc_scheme* scheme, int32_t checkpoint_every,
+                               const mc_allocator* memory, mc_adjoint** out) {
     if (!grid || !scheme || !out || checkpoint_every < 1) {
         return afail(MC_ERR_INVALID_ARGUMENT, "null argument or checkpoint interval < 1");
     }
     *out = nullptr;
+    if (memory && (!memory->alloc || !memory->free)) {
+        return afail(MC_ERR_INVALID_ARGUMENT, "an allocator needs alloc and free");
+    }
     const mc_grid& g = *grid;
     const mc_scheme& s = *scheme;
     if (g.num_dim != 2 || g.num_tracers != 0 || s.reconstruction != MC_RECON_WENO5Z ||
@@ -751,6 +776,9 @@ mc_status mc_adjoint_create(const mc_grid* grid, const mc_scheme* scheme, int32_
         return afail(MC_ERR_OUT_OF_MEMORY, "host allocation");
     }
     cudaGetDevice(&a->device);
+    if (memory) {
+        a->memory = *memory;
+    }
     a->grid = g;
     a->scheme = s;
     a->k = checkpoint_every;
@@ -794,19 +822,7 @@ mc_status mc_adjoint_destroy(mc_adjoint* a) {
     if (!a) {
         return MC_OK;
     }
-    // the blocks may be handed to another adjoint: nothing may still use them
-    int device = a->device;
-    cudaGetDevice(&device);
-    cudaSetDevice(a->device);
-    const bool idle = cudaDeviceSynchronize() == cudaSuccess;
-    for (const auto& b : a->blocks) {
-        if (idle) {
-            mc::block_free(b.first, b.second, a->device);
-        } else {
-            cudaFree(b.first);
-        }
-    }
-    cudaSetDevice(device);
+    free_blocks(a, {}, true);
     mc::slab_destroy(a->slab);
     delete a;
     return MC_OK;

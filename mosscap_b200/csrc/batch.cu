@@ -11,7 +11,6 @@
 #include <string>
 #include <vector>
 
-#include "blocks.h"
 #include "batch_launch.h"
 #include "launch.h"
 #include "mosscap_b200.h"
@@ -419,7 +418,7 @@ mc_status mc_batch_create(const mc_batch_problem* problems, int32_t n, const mc_
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void** p, size_t bytes) {
         if (e == cudaSuccess) {
-            e = mc::device_alloc(p, bytes);
+            e = cudaMalloc(p, bytes);
         }
     };
     alloc((void**)&b->buf_a, sizeof(double) * (size_t)pool_doubles);

@@ -12,7 +12,6 @@
 #include <string>
 #include <vector>
 
-#include "blocks.h"
 #include "eos.h"
 #include "launch.h"
 #include "mosscap_b200.h"
@@ -771,12 +770,12 @@ mc_status mc_create(const mc_grid* grid, const mc_scheme* scheme, mc_ctx** out) 
     c->nvar = 2 + g.num_dim + g.num_tracers;
     c->plane = (long long)g.xc * g.yc * g.zc;
     c->state_bytes = sizeof(double) * (size_t)c->nvar * (size_t)c->plane;
-    cudaError_t e = mc::device_alloc((void**)&c->buf_a, c->state_bytes);
+    cudaError_t e = cudaMalloc(&c->buf_a, c->state_bytes);
     if (e == cudaSuccess) {
-        e = mc::device_alloc((void**)&c->buf_b, c->state_bytes);
+        e = cudaMalloc(&c->buf_b, c->state_bytes);
     }
     if (e == cudaSuccess && g.num_dim == 3) {
-        e = mc::device_alloc((void**)&c->dqxy, sizeof(double) * (size_t)c->nvar * c->nx * c->ny * c->nz);
+        e = cudaMalloc(&c->dqxy, sizeof(double) * (size_t)c->nvar * c->nx * c->ny * c->nz);
     }
     if (e == cudaSuccess) {
         e = cudaMalloc(&c->blk, sizeof(mc::DeviceBlock));
