@@ -17,17 +17,17 @@
 
 namespace mc {
 
-// 1 / d for the reverse sweep: the PTX approximation r0 = rcp.approx.ftz.f64 =
-// (1 - e) / d, |e| <= 2^-19.9, and r = r0 (1 + e + e^2), short of 1 / d by e^3 and the last
-// rounding: three FP64 instructions (two Newton steps take four: backward of 20 steps on
-// 512^2 9.88 -> 9.75 ms). For normal d with a normal reciprocal (every denominator here:
-// densities, pressures, sound speeds, the WENO weight sums, regularised smoothness
-// indicators and HLLC wave-speed differences).
+// 1 / d for the reverse sweep: the PTX approximation rcp.approx.ftz.f64
+// refined by two Newton-Raphson steps r <- r + r (1 - d r), each of which
+// squares the relative error. For normal d with a normal reciprocal (every
+// denominator here: densities, pressures, sound speeds, the WENO weight sums,
+// regularised smoothness indicators and HLLC wave-speed differences).
 __device__ __forceinline__ double arcp(double d) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
     double e = fma(-d, r, 1.0);
-    e = fma(e, e, e);
+    r = fma(r, e, r);
+    e = fma(-d, r, 1.0);
     return fma(r, e, r);
 }
 
