@@ -19,7 +19,9 @@ namespace mc {
 
 // 1 / d for the reverse sweep: the PTX approximation rcp.approx.ftz.f64
 // refined by two Newton-Raphson steps r <- r + r (1 - d r), each of which
-// squares the relative error. For normal d with a normal reciprocal (every
+// squares the relative error (2^-80 before the last rounding; one third-order step is an
+// instruction shorter, backward of 20 steps on 512^2 9.88 -> 9.75 ms, but leaves 2^-59.8:
+// not taken). For normal d with a normal reciprocal (every
 // denominator here: densities, pressures, sound speeds, the WENO weight sums,
 // regularised smoothness indicators and HLLC wave-speed differences).
 __device__ __forceinline__ double arcp(double d) {
