@@ -506,6 +506,13 @@ mc_status mc_debug_reverse_reciprocal(const double* x, double* out, int64_t n, v
  * counterpart in the reference. */
 mc_status mc_debug_exact_ops(int32_t op, const double* a, const double* b, double* out, int64_t n, void* stream);
 
+/* Diagnostic: y and T (n doubles each) of a 1D state q ([3][n]) by the
+ * analytic LTE hydrogen update, or (plain) with the bisection's function
+ * evaluated at every step, so that the two can be compared on one device. No
+ * counterpart in the reference. */
+mc_status mc_debug_lte_update(const double* q, int64_t n, double gamma, double avg_mass, int32_t ionisation,
+                              int32_t plain, double* y, double* T, void* stream);
+
 /* Message of the last failed call on this thread (static storage). */
 const char* mc_last_error(void);
 

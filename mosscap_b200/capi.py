@@ -208,6 +208,8 @@ def load() -> ctypes.CDLL:
     lib.mc_debug_reverse_reciprocal.restype = i32
     lib.mc_debug_exact_ops.argtypes = [i32, vp, vp, vp, i64, vp]
     lib.mc_debug_exact_ops.restype = i32
+    lib.mc_debug_lte_update.argtypes = [vp, i64, d, d, i32, i32, vp, vp, vp]
+    lib.mc_debug_lte_update.restype = i32
     if lib.mc_abi_version() != 1:
         raise RuntimeError("unexpected ABI version")
     _LIB = lib

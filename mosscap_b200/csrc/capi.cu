@@ -1284,6 +1284,29 @@ mc_status mc_debug_exact_ops(int32_t op, const double* a, const double* b, doubl
     return MC_OK;
 }
 
+mc_status mc_debug_lte_update(const double* q, int64_t n, double gamma, double avg_mass, int32_t ionisation,
+                              int32_t plain, double* y, double* T, void* stream) {
+    if (!q || !y || !T || n < 0 || !(avg_mass > 0.0)) {
+        return fail(MC_ERR_INVALID_ARGUMENT, "null argument, negative count or avg_mass <= 0");
+    }
+    mc::EosLaunch L{};
+    L.type = mc::kEosAnalytic;
+    L.q_in = q;
+    L.y = y;
+    L.T = T;
+    L.plane = n;
+    L.nvar = 3;
+    L.gamma = gamma;
+    L.avg_mass = avg_mass;
+    L.ionisation_e = ionisation ? 1 : 0;
+    if (n > 0) {
+        MC_CUDA(plain ? mc::launch_eos_analytic_plain(L, (cudaStream_t)stream)
+                      : mc::launch_eos_update(L, 1, (cudaStream_t)stream),
+                "LTE update");
+    }
+    return MC_OK;
+}
+
 int64_t mc_launch_count(const mc_ctx* c) {
     return c ? c->launches : 0;
 }

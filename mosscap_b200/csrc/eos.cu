@@ -30,14 +30,64 @@ constexpr double kHMass = 1.6737830080950003e-27;  // [kg]
 constexpr double kKB = 1.380649e-23;               // [J / K]
 constexpr double kChiH = 2.178710282685096e-18;    // [J]
 
-__device__ __forceinline__ double saha_rhs_H(double temp) {
-    return 2.4146830395719654e+21 * pow(temp, 1.5) * exp(-157763.42386247337 / temp);
+// IEEE division and the ionisation fraction with it, for operands outside exact_fp64.cuh's.
+__device__ __noinline__ double div_any(double a, double b) {
+    return a / b;
 }
-
-__device__ __forceinline__ double y_from_nhtot(double nhtot, double temp) {
-    const double X = saha_rhs_H(temp);
+__device__ __noinline__ double y_any(double nhtot, double X) {
     return 0.5 * (-X + sqrt(X * X + 4 * nhtot * X)) / nhtot;
 }
+
+// Positive and in [2^-400, 2^340).
+__device__ __forceinline__ bool lte_range(double x) {
+    return (unsigned)(__double2hiint(x) - 0x26f00000) < 0x55300000u - 0x26f00000u;
+}
+
+// One cell's F(T) = T - T(y(T)) and its y (source/AnalyticLteH.hpp:49-76). With !PLAIN the
+// quotients and the root are exact_fp64.cuh's, for operands that meet its conditions: X,
+// e_to_T and T in lte_range and n in it above 2^-40. Then -X + sqrt(X^2 + 4 n X) is zero or
+// at least an ulp of X, 2^-452, and y, rounding errors of that included, below 2^330. The
+// same bits.
+template <bool PLAIN>
+struct LteCell {
+    double nhtot, e_to_T, eint, rho, inv_avg_mass;
+    double ion_e;  // 1 with the ionisation energy, 0 without
+    Recip rn;
+    bool n_ok, e_ok;
+    __device__ __forceinline__ LteCell(double rho_, double nhtot_, double e_to_T_, double eint_, double ion_e_,
+                                       double inv_avg_mass_) {
+        rho = rho_;
+        nhtot = nhtot_;
+        e_to_T = e_to_T_;
+        eint = eint_;
+        ion_e = ion_e_;
+        inv_avg_mass = inv_avg_mass_;
+        n_ok = !PLAIN && lte_range(nhtot) && nhtot >= 0x1p-40;
+        e_ok = !PLAIN && lte_range(e_to_T);
+        rn = recip_of(nhtot);
+    }
+    // small: y is below 2^330
+    __device__ __forceinline__ double temp_from_y(double y, bool small) const {
+        const double d = 1.0 + y;
+        const double t = e_ok && small ? exact_div(e_to_T, d) : PLAIN ? e_to_T / d : div_any(e_to_T, d);
+        return t * (eint - ion_e * y * rho * (kChiH / kHMass) * inv_avg_mass);
+    }
+    __device__ __forceinline__ double f_of(double temp, double& y) const {
+        bool small;
+        y = y_of(temp, small);
+        return temp - temp_from_y(y, small);
+    }
+    __device__ __forceinline__ double y_of(double temp, bool& small) const {
+        const double chi = -157763.42386247337;
+        const double a = !PLAIN && lte_range(temp) ? exact_div(chi, temp) : PLAIN ? chi / temp : div_any(chi, temp);
+        const double X = 2.4146830395719654e+21 * pow(temp, 1.5) * exp(a);
+        small = n_ok && lte_range(X);
+        if (small) {
+            return exact_quot(0.5 * (-X + exact_sqrt(X * X + 4 * nhtot * X)), rn);
+        }
+        return PLAIN ? 0.5 * (-X + sqrt(X * X + 4 * nhtot * X)) / nhtot : y_any(nhtot, X);
+    }
+};
 
 template <int NDIM>
 __device__ __forceinline__ void energies(const double* q, long long id, long long plane, double& rho, double& e_kin,
@@ -60,7 +110,7 @@ __device__ __forceinline__ void energies(const double* q, long long id, long lon
 // slope: F' there.
 __device__ __forceinline__ float lte_root_estimate(float t0, float t1, float c, float k, float& slope) {
     float lo = t0, hi = t1, t = 0.5f * (t0 + t1);
-    for (int it = 0; it < 8; ++it) {
+    for (int it = 0; it < 16; ++it) {
         const float it_ = __fdividef(1.0f, t);
         const float r = c * t * __fsqrt_rn(t) * __expf(-157763.42f * it_);
         const float y = __fdividef(2.0f, 1.0f + __fsqrt_rn(1.0f + __fdividef(4.0f, r)));
@@ -84,43 +134,70 @@ __device__ __forceinline__ float lte_root_estimate(float t0, float t1, float c, 
     return t;
 }
 
+// A cell's F and how far its evaluation in FP64 can be off, all in FP32: amp = t1 (1 + k) and
+// c of lte_root_estimate. The evaluation's error at T is at most
+// u t1 (1 + k) ((r + 2) / (1 + y)^2 + 5 + (10 + 157763.4 / T) y (1 - y) / ((2 - y) (1 + y)^2)),
+// u = 2^-53, r = X / n = c T^1.5 exp(-157763.4 / T): dT/dy = -t1 (1 + k) / (1 + y)^2 times
+// y's error, which is that of -X + sqrt(X^2 + 4 n X) (sqrt's argument off by 2 u, its own
+// rounding u: u (X + 2 n) / n) and that of X itself (pow, exp and its argument), and
+// temp_from_y's own roundings. With 1 + y >= (1 + 2 r) / (1 + r), T >= 100 and the last
+// fraction at most 0.08 it is below u amp (r / 4 + 160), which grows with T.
+constexpr float kLteErrorMax = 0.0045f;  // [K]; twice this is below the replay's margin of 0.01
+struct LteError {
+    float amp, c;
+    __device__ __forceinline__ float operator()(float T) const {
+        const float r = c * (T * T) * rsqrtf(T) * __expf(__fdividef(-157763.42f, T));
+        return 1.1103e-16f * amp * (0.25f * r + 160.0f);
+    }
+    // Whether the error stays within the limit from `hi` up to where F is large, for tests up to t1.
+    __device__ __forceinline__ bool allows(float hi, float t1) const {
+        return (*this)(fminf(hi + 1.0f + (*this)(t1), t1)) < kLteErrorMax;
+    }
+};
+
 // The reference's bisection (source/AnalyticLteH.hpp:78-119) halves [T(y = 1), T(y = 0)]
 // about 17 times, with a pow, an exp and a root for each test temperature: FP64-bound. Its
 // outcome is fixed by the signs of F(T) = T - T(y(T)) at the test temperatures and by
 // whether |F| < 0.1 there. F' >= 1 (y grows with T, and T(y) falls with y), so one value
 // F(r) bounds the root: it lies between r and r - F(r); and a test temperature more than
-// 0.1 beyond that bracket (0.11, for rounding) has a known sign and |F| > 0.1. So the
-// bisection is replayed, and F evaluated, with the same expressions, only at an FP32
-// estimate of the root, at the test temperatures near it and at the last one (whose y is
-// the result): 2.3 evaluations per cell where it took 15 (1e-9 .. 1e-6 kg/m^3, 5e3 .. 2e4 K;
-// 3.3 and 18 with the ionisation energy). Cells outside the argument (non-positive or
-// non-finite density or energy, flipped bounds, rounding errors of F near the root that the
-// margin does not cover) are evaluated at every step.
-// One update of 512^2 smooth cells (B200): 70 -> 33 us around 1e4 K and 3e-8 kg/m^3, 84 -> 80
-// with the ionisation energy, 63 -> 27 us around 5e3 K and 1e-4; 102 -> 105 us at 1e6 K and
-// 1e-12, where F is all rounding error and every step is evaluated.
-template <int NDIM>
-__global__ void __launch_bounds__(256) eos_analytic_kernel(EosLaunch L) {
+// 0.1 beyond that bracket has a known sign and |F| > 0.1. So the bisection is replayed, and
+// F evaluated, with the same expressions, only at an FP32 estimate of the root, at the test
+// temperatures near it and at the last one (whose y is the result): 2.3 evaluations per cell
+// where it took 15 (1e-9 .. 1e-6 kg/m^3, 5e3 .. 2e4 K; 3.3 and 18 with the ionisation energy).
+// Both values are evaluated with an error: 0.11 in place of 0.1 leaves 0.01 for that of the
+// bracket's and that of the skipped one together. Each bracketing evaluation is at a
+// temperature where the error is at most kLteErrorMax, and it must stay so up to hi + 1 +
+// its largest value, beyond which F exceeds it by more than 0.1 in any case. Cells that
+// do not meet this, and those outside the argument (non-positive or non-finite density or
+// energy, flipped bounds), are evaluated at every step.
+// PLAIN: every cell is (the same bits; for comparison).
+// One update of 512^2 smooth cells (B200), IEEE divisions and every step evaluated -> this
+// kernel: 68 -> 33 us around 1e4 K and 3e-8 kg/m^3, 83 -> 75 with the ionisation energy; 62 ->
+// 27 and 64 -> 28 around 5e3 K and 1e-4; where F is mostly rounding error and no bracket is
+// allowed 101 -> 97 and 101 -> 97 (1e6 K, 1e-12), 78 -> 76 and 85 -> 86 (4e4 K, 1e-10), 83 -> 82
+// and 87 -> 87 (1e5 K, 1e-8). Four CTAs per SM: the registers of three take 91 us in the second.
+template <int NDIM, bool PLAIN = false>
+__global__ void __launch_bounds__(256, 4) eos_analytic_kernel(EosLaunch L) {
     if (L.blk && L.skip_when_done && L.blk->done) {
         return;
     }
     const double gamma = L.gamma;
     const double ionisation_e = L.ionisation_e ? 1.0 : 0.0;
     const double inv_avg_mass = 1.0 / L.avg_mass;
+    // t1 k of lte_root_estimate: the same for every cell
+    const float t1k = L.ionisation_e ? (float)(kChiH / kKB * (gamma - 1.0)) : 0.0f;
     unsigned flags = 0;
     for (long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x; id < L.plane;
          id += (long long)gridDim.x * blockDim.x) {
         double rho, e_kin, eint;
         energies<NDIM>(L.q_in, id, L.plane, rho, e_kin, eint);
         const double e_to_T = (gamma - 1.0) / (rho * (kKB / kHMass) * inv_avg_mass);
-        auto temp_from_y = [&](double y) {
-            return e_to_T / (1.0 + y) * (eint - ionisation_e * y * rho * (kChiH / kHMass) * inv_avg_mass);
-        };
-        const double rho_to_nhtot = (1.0 / kHMass) * inv_avg_mass;
+        const double nhtot = rho * ((1.0 / kHMass) * inv_avg_mass);
+        const LteCell<PLAIN> cell(rho, nhtot, e_to_T, eint, ionisation_e, inv_avg_mass);
         const double min_temperature = 100.0;
-        const double t1 = temp_from_y(1.0);
+        const double t1 = cell.temp_from_y(1.0, true);
         const double tb0 = (t1 < min_temperature) ? min_temperature : t1;  // std::max
-        const double tb1 = temp_from_y(0.0);
+        const double tb1 = cell.temp_from_y(0.0, true);
         if (tb0 > tb1) {
             flags |= kFlagEos;
         }
@@ -130,32 +207,30 @@ __global__ void __launch_bounds__(256) eos_analytic_kernel(EosLaunch L) {
         // the root's bracket; (-inf, inf): every test temperature is evaluated
         double lo = -__longlong_as_double(0x7ff0000000000000ll), hi = -lo;
         double test_temp = 0.0;
+        LteError error{0.0f, 0.0f};
         float slope = 1.0f;
         bool bracket = false;
         int iter = 0;  // tests so far; negative: evaluations for the bracket
-        if (rho > 0.0 && eint > 0.0 && e_to_T > 0.0 && tb1 > tb0) {
-            const float c = (float)(2.4146830395719654e+21 / (rho * rho_to_nhtot));
-            const float k = (float)(ionisation_e * rho * (kChiH / kHMass) * inv_avg_mass / eint);
-            // F's rounding error, mostly that of -X + sqrt(X^2 + 4 n X), is at most
-            // 4e-17 T X(T) / n: it must stay below a fifth of the margin from the root up
-            // to where the distance from the root is four times its largest value
-            auto error = [&](float T) { return 4e-17f * T * c * T * __fsqrt_rn(T) * __expf(__fdividef(-157763.42f, T)); };
-            if (error((float)tb0) < 0.002f) {
-                const float root = lte_root_estimate((float)tb0, (float)tb1, c, k, slope);
-                if (error(root + 4.0f * error((float)tb1) + 1.0f) < 0.002f) {
+        const float nf = (float)nhtot, t0f = (float)tb0, t1f = (float)tb1;
+        // (density and, tb0 being at least 100, energy are positive)
+        if (!PLAIN && gamma > 1.0 && nf > 0.0f && t1f > t0f) {
+            error.amp = t1f + t1k;
+            error.c = __fdividef(2.4146830e21f, nf);
+            if (error(t0f) < kLteErrorMax) {
+                const float root = lte_root_estimate(t0f, t1f, error.c, __fdividef(t1k, t1f), slope);
+                if (error(root) < kLteErrorMax && error.allows(root, t1f)) {
                     test_temp = (double)root;
                     bracket = true;
                     iter = -2;
                 }
             }
         }
-        if (!__any_sync(__activemask(), bracket)) {
+        if (PLAIN || !__any_sync(__activemask(), bracket)) {
             // no lane has a bracket: the plain loop
-            for (; iter < 100; ++iter) {
+            for (iter = 0; iter < 100; ++iter) {
                 temp_step *= 0.5;
                 test_temp = temp + temp_step;
-                y = y_from_nhtot(rho * rho_to_nhtot, test_temp);
-                const double temp_err = test_temp - temp_from_y(y);
+                const double temp_err = cell.f_of(test_temp, y);
                 if (temp_err <= 0.0) {
                     temp = test_temp;
                 }
@@ -183,8 +258,8 @@ __global__ void __launch_bounds__(256) eos_analytic_kernel(EosLaunch L) {
                     }
                 }
             }
-            const double yt = y_from_nhtot(rho * rho_to_nhtot, test_temp);
-            const double temp_err = test_temp - temp_from_y(yt);
+            double yt;
+            const double temp_err = cell.f_of(test_temp, yt);
             if (bracket && temp_err > 0.0) {
                 hi = test_temp < hi ? test_temp : hi;
                 lo = test_temp - temp_err > lo ? test_temp - temp_err : lo;
@@ -195,8 +270,18 @@ __global__ void __launch_bounds__(256) eos_analytic_kernel(EosLaunch L) {
             if (iter < 0) {
                 // a steep F leaves a wide bracket: once more, somewhat beyond the
                 // Newton step from here, where F mostly has the other sign
-                iter = (iter == -2 && fabs(temp_err) > 0.1) ? -1 : 0;
-                test_temp -= 1.5 * temp_err / (double)slope;
+                const double next = test_temp - 1.5 * temp_err / (double)slope;
+                if (iter == -2 && fabs(temp_err) > 0.1 && error((float)next) < kLteErrorMax) {
+                    iter = -1;
+                    test_temp = next;
+                    continue;
+                }
+                iter = 0;
+                if (!error.allows((float)hi, t1f)) {
+                    bracket = false;
+                    hi = __longlong_as_double(0x7ff0000000000000ll);
+                    lo = -hi;
+                }
                 continue;
             }
             y = yt;
@@ -361,6 +446,12 @@ cudaError_t allow_table_smem(K kernel, size_t bytes) {
 }
 
 } // namespace
+
+cudaError_t launch_eos_analytic_plain(const EosLaunch& L, cudaStream_t s) {
+    const long long want = (L.plane + 255) / 256;
+    eos_analytic_kernel<1, true><<<(int)(want < 148 * 16 ? want : 148 * 16), 256, 0, s>>>(L);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_eos_update(const EosLaunch& L, int ndim, cudaStream_t s) {
     const long long want = (L.plane + 255) / 256;

@@ -31,6 +31,8 @@ struct EosLaunch {
     int skip_when_done;
 };
 
+// The analytic update of a 1D state with F evaluated at every step of the bisection.
+cudaError_t launch_eos_analytic_plain(const EosLaunch& L, cudaStream_t s);
 cudaError_t launch_eos_update(const EosLaunch& L, int ndim, cudaStream_t s);
 
 } // namespace mc
