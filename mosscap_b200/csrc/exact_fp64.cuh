@@ -94,7 +94,8 @@ __device__ __forceinline__ Recip recip_of(double b) {
 
 // RN(a / b) for b whose reciprocal is normal and a that is zero (the result is a
 // zero of either sign: no result of the stage kernels depends on it) or so
-// that the quotient is normal and |a| > 2^-900.
+// that the quotient is normal and |a| > 2^-960 (the residual's last bit, 2^-106 of a, is
+// then a double).
 __device__ __forceinline__ double exact_quot(double a, const Recip& r) {
     const double t = __dmul_rn(a, r.y);
     const double q = fma(t, r.s, t);
@@ -123,19 +124,43 @@ __device__ __forceinline__ double exact_sqrt(double x) {
 // ---- Range tests -------------------------------------------------------------
 //
 // A cell is in range when rho and p lie in [2^-120, 2^100) and each velocity
-// and mass fraction is zero or of magnitude in [2^-250, 2^100). Then every
-// division and root below meets its conditions: sums and products of such
-// values that are not zero are at least 2^-303 (an operand's last bit), WENO
-// weights at least 1 and at most 2^650, and so on; the face states a
-// reconstruction makes of them are tested again before the Riemann solver
-// (positivity is not kept by it). Upper words as integers: one or two
-// instructions of the integer pipe for each value, none of the FP64 pipe.
+// and mass fraction is zero or of magnitude in [2^-800, 2^100) ([2^-420, 2^100) where
+// a van Leer slope multiplies two of their differences). Then every division and root
+// below meets its conditions or its result does not matter:
+//   a momentum that is not zero is at least 2^-920, and differences of such velocities
+//   are zero or at least an operand's last bit, 2^-852 (2^-472: their products 2^-944);
+//   factors 2 and fmas in place of products with a power of two are exact at these sizes;
+//   WENO5-Z: squares of differences below 2^-537 vanish, as in physics.cuh, beside the
+//   regulariser 2^-119.6; the weights are at least 1 and at most 2^650; the weighted sum is
+//   zero or at least 2^-904, and its quotient by the weights' sum normal: if the sum is
+//   large, the smooth substencil's own term, or, where that is zero, a large cell's, is too;
+//   kinetic energies, momentum fluxes and wave-speed terms of velocities this small are
+//   formed by the same operations as in physics.cuh, or vanish beside p >= 2^-120.
+// The face states a reconstruction makes of them are tested again before the Riemann solver
+// (positivity is not kept by it). Upper words as integers: one or two instructions of
+// the integer pipe for each value, none of the FP64 pipe.
+// Velocities decay to nothing ahead of a front in a uniform medium, so their bound is as low
+// as this allows: KH 2048^2 with the velocities across the flow times 1e-200, WENO5-Z, 2.64
+// -> 1.40 ms per step against a bound of 2^-250. Denormal ones stay out: Sedov 256^3 has
+// them in 5 to 7 % of its tiles from step 20 on and takes 2.4 % longer there than before.
+constexpr unsigned kVelLow = 0x0df00000u;         // upper word of 2^-800
+constexpr unsigned kVelLowVanLeer = 0x25b00000u;  // 2^-420
+template <int REC, int LIM>
+__host__ __device__ constexpr unsigned vel_low() {
+    return LIM == kVanLeer && (REC == kMuscl || REC == kPpm) ? kVelLowVanLeer : kVelLow;
+}
 __device__ __forceinline__ bool in_range_pos(double x) {
     return (unsigned)(__double2hiint(x) - 0x38700000) < 0x46300000u - 0x38700000u;
 }
-__device__ __forceinline__ bool in_range_any(double x) {
-    const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
-    return hi - 0x30500000u < 0x46300000u - 0x30500000u || (hi | (unsigned)__double2loint(x)) == 0u;
+template <unsigned LOW>
+__device__ __forceinline__ bool in_range_magnitude(double x) {
+    return ((unsigned)__double2hiint(x) & 0x7fffffffu) - LOW < 0x46300000u - LOW;
+}
+// x, a quotient with numerator n.
+template <unsigned LOW>
+__device__ __forceinline__ bool in_range_any(double x, double n) {
+    return in_range_magnitude<LOW>(x) ||
+           (((unsigned)__double2hiint(n) & 0x7fffffffu) | (unsigned)__double2loint(n)) == 0u;
 }
 // Four upper words of positive values at once.
 __device__ __forceinline__ bool in_range_pos4(double a, double b, double c, double d) {
@@ -163,7 +188,7 @@ inline FastGas fast_gas(double gamma) {
 // ---- physics.cuh's functions for values in range -------------------------------
 
 // prim_from_cons; false: the cell is out of range and w holds no result.
-template <int NDIM>
+template <int NDIM, unsigned LOW>
 __device__ __forceinline__ bool fast_prim(double gm1, const double* q, double* w) {
     const Recip r = recip_of(q[0]);
     w[0] = q[0];
@@ -171,16 +196,25 @@ __device__ __forceinline__ bool fast_prim(double gm1, const double* q, double* w
     for (int d = 1; d <= NDIM; ++d) {
         w[d] = exact_quot(q[d], r);
     }
-    bool ok = in_range_pos(q[0]);
+    bool ok = true;
     double v2 = 0.0;
 #pragma unroll
     for (int d = 1; d <= NDIM; ++d) {
-        ok = ok && in_range_any(w[d]);
+        ok = ok && in_range_magnitude<LOW>(w[d]);
         v2 = d == 1 ? __dmul_rn(w[d], w[d]) : __dadd_rn(v2, __dmul_rn(w[d], w[d]));
     }
     // E - (0.5 rho) v2: the factor 1/2 is exact
     w[1 + NDIM] = __dmul_rn(gm1, fma(-0.5, __dmul_rn(q[0], v2), q[1 + NDIM]));
-    return ok && in_range_pos(w[1 + NDIM]);
+    if (!ok) {
+        // velocities that are zero, by their momenta (a quotient may vanish beside a momentum
+        // that does not; tested here and not for every cell: KH 2048^2 step -0.4 %)
+        ok = true;
+#pragma unroll
+        for (int d = 1; d <= NDIM; ++d) {
+            ok = ok && in_range_any<LOW>(w[d], q[d]);
+        }
+    }
+    return ok && in_range_pos(q[0]) && in_range_pos(w[1 + NDIM]);
 }
 
 // cfl_dt of a cell in range.
@@ -194,7 +228,8 @@ __device__ __forceinline__ double fast_cfl_dt(double gamma, double dx, const dou
     if constexpr (NDIM > 2) {
         v2 = __dadd_rn(v2, __dmul_rn(w[3], w[3]));
     }
-    const double vel = v2 == 0.0 ? 0.0 : exact_sqrt(v2);
+    // v2 below 2^-900 leaves cs + |v| = cs
+    const double vel = __double2hiint(v2) < 0x07b00000 ? 0.0 : exact_sqrt(v2);
     return exact_div(dx, __dadd_rn(cs, vel));
 }
 

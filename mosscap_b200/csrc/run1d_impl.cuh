@@ -112,7 +112,7 @@ __device__ __forceinline__ void run_segment(const StageParams& p, bool last, int
             }
         }
         double w[nh];
-        const bool ok = prim_for_sweep<NDIM, Real>(p.gamma, p.gas, q, w);
+        const bool ok = prim_for_sweep<NDIM, Real, vel_low<REC, LIM>()>(p.gamma, p.gas, q, w);
         in_range = in_range && ok;
 #pragma unroll
         for (int v = 0; v < nh; ++v) {
@@ -125,7 +125,7 @@ __device__ __forceinline__ void run_segment(const StageParams& p, bool last, int
                 if (t < p.ntracer) {
                     const Real s = Real(q[nh + t] * inv_rho);
                     W[(nh + t) * WN + it] = s;
-                    in_range = in_range && (sizeof(Real) == 4 || in_range_any(s));
+                    in_range = in_range && (sizeof(Real) == 4 || in_range_any<vel_low<REC, LIM>()>(s, s));
                 }
             }
         }

@@ -115,7 +115,7 @@ __device__ __forceinline__ double cfl_bound_of(const StageParams& p, const doubl
     constexpr int nh = 2 + NDIM;
     if constexpr (sizeof(T) == 8) {
         double w[nh];
-        if (p.gas.ok && in_range_pos(p.dx) && fast_prim<NDIM>(p.gas.gm1, q, w)) {
+        if (p.gas.ok && in_range_pos(p.dx) && fast_prim<NDIM, kVelLow>(p.gas.gm1, q, w)) {
             return fast_cfl_dt<NDIM>(p.gamma, p.dx, w);  // in range: no flag to raise
         }
     }
@@ -328,10 +328,10 @@ __device__ __forceinline__ double write_cell(const StageParams& p, int i, int j,
 // near-vacuum cells stays an FP64 operation -- one FP64 division per cell
 // instead of 2 + (NDIM > 1) + (NDIM > 2).
 // Returns whether the cell is in range for the FP64 sweep (exact_fp64.cuh).
-template <int NDIM, class T>
+template <int NDIM, class T, unsigned LOW>
 __device__ __forceinline__ bool prim_for_sweep(double gamma, const FastGas& gas, const double* q, double* w) {
     if constexpr (sizeof(T) == 8) {
-        const bool ok = fast_prim<NDIM>(gas.gm1, q, w);
+        const bool ok = fast_prim<NDIM, LOW>(gas.gm1, q, w);
         if (!ok) {
             prim_from_cons<NDIM>(gamma, q, w);
         }
@@ -379,12 +379,12 @@ __device__ __forceinline__ void load_cons(const StageParams& p, int k, int j, in
 // Store the primitives of the cell whose conserved variables load_cons read
 // (tracers, loaded here, divided by rho, source/Hydro.cpp:27-33) into shared memory.
 // Clears in_range unless the cell is in range for the FP64 sweep.
-template <int NDIM, class T>
+template <int NDIM, class T, unsigned LOW>
 __device__ __forceinline__ unsigned store_prim(const StageParams& p, int k, int j, int i, bool inb, const double* q,
                                                T* w_smem, int var_stride, bool& in_range) {
     constexpr int nh = 2 + NDIM;
     double w[nh];
-    const bool ok = prim_for_sweep<NDIM, T>(p.gamma, p.gas, q, w);
+    const bool ok = prim_for_sweep<NDIM, T, LOW>(p.gamma, p.gas, q, w);
     in_range = in_range && ok;
 #pragma unroll
     for (int v = 0; v < nh; ++v) {
@@ -399,7 +399,7 @@ __device__ __forceinline__ unsigned store_prim(const StageParams& p, int k, int 
             const T s = T(qt * inv_rho);
             w_smem[(nh + t) * var_stride] = s;
             if constexpr (sizeof(T) == 8) {
-                in_range = in_range && in_range_any(s);
+                in_range = in_range && in_range_any<LOW>(s, s);
             }
         }
     }
@@ -414,17 +414,17 @@ __device__ __forceinline__ unsigned store_prim(const StageParams& p, int k, int 
     return state_flags(w[0], w[nh - 1], fin);
 }
 
-template <int NDIM, class T>
+template <int NDIM, class T, unsigned LOW>
 __device__ __forceinline__ unsigned load_prim(const StageParams& p, int k, int j, int i, bool inb, T* w_smem,
                                               int var_stride, bool& in_range) {
     double q[2 + NDIM];
     load_cons<NDIM>(p, k, j, i, inb, q);
-    return store_prim<NDIM, T>(p, k, j, i, inb, q, w_smem, var_stride, in_range);
+    return store_prim<NDIM, T, LOW>(p, k, j, i, inb, q, w_smem, var_stride, in_range);
 }
 
 // The same as load_prim for a cell whose conserved variables sit in the
 // TMA-staged tile (variable stride stg_vs doubles); no tracers.
-template <int NDIM, class T>
+template <int NDIM, class T, unsigned LOW>
 __device__ __forceinline__ unsigned staged_prim(const StageParams& p, const double* src, int stg_vs, bool inb,
                                                 T* w_smem, int var_stride, bool& in_range) {
     constexpr int nh = 2 + NDIM;
@@ -443,7 +443,7 @@ __device__ __forceinline__ unsigned staged_prim(const StageParams& p, const doub
         }
         q[nh - 1] = 1.0;
     }
-    const bool ok = prim_for_sweep<NDIM, T>(p.gamma, p.gas, q, w);
+    const bool ok = prim_for_sweep<NDIM, T, LOW>(p.gamma, p.gas, q, w);
     in_range = in_range && ok;
 #pragma unroll
     for (int v = 0; v < nh; ++v) {
@@ -710,7 +710,7 @@ __device__ __forceinline__ void segment1d(const StageParams& p, int x0, T* W, do
     for (int it = lane; it < WN; it += 32) {
         const int i = p.ng + x0 - H + it;  // array index
         const bool inb = i >= 0 && i < p.xc;
-        flags |= load_prim<NDIM, T>(p, 0, 0, i, inb, W + it, WN, in_range);
+        flags |= load_prim<NDIM, T, vel_low<REC, LIM>()>(p, 0, 0, i, inb, W + it, WN, in_range);
     }
     __syncwarp();
     in_range = __all_sync(0xffffffffu, in_range);
@@ -884,7 +884,7 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
             const int i = p.ng + x0 + tx;
             const int j = p.ng + y0 + ty;
             const bool inb = i >= 0 && i < p.xc && j >= 0 && j < p.yc;
-            flags |= staged_prim<NDIM, T>(p, stg + (ty + H) * SX + (tx + H + xo), SX * (th + 2 * H), inb,
+            flags |= staged_prim<NDIM, T, vel_low<REC, LIM>()>(p, stg + (ty + H) * SX + (tx + H + xo), SX * (th + 2 * H), inb,
                                           W + (ty + H) * P + (tx + H), WV, in_range);
         }
     } else {
@@ -934,7 +934,7 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
                 const int i = p.ng + x0 + tx;
                 const int j = p.ng + y0 + ty;
                 const bool inb = i >= 0 && i < p.xc && j >= 0 && j < p.yc;
-                flags |= store_prim<NDIM, T>(p, k, j, i, inb, q[u], W + (ty + H) * P + (tx + H), WV, in_range);
+                flags |= store_prim<NDIM, T, vel_low<REC, LIM>()>(p, k, j, i, inb, q[u], W + (ty + H) * P + (tx + H), WV, in_range);
             }
         }
     }
@@ -1329,7 +1329,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks2d)
             const int x = it - r * kZCols;
             const int k = p.ng + z0 - H + r;
             const bool inb = x < vw && k >= 0 && k < p.zc;
-            flags |= staged_prim<NDIM, T>(p, stg + r * kZStageX + x + xoff, SV, inb, W + r * PZ + x, WV,
+            flags |= staged_prim<NDIM, T, vel_low<REC, LIM>()>(p, stg + r * kZStageX + x + xoff, SV, inb, W + r * PZ + x, WV,
                                           in_range);
         }
     } else {
@@ -1339,7 +1339,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks2d)
             const int i = p.ng + x0 + x;
             const int k = p.ng + z0 - H + r;
             const bool inb = x < vw && k >= 0 && k < p.zc;
-            flags |= load_prim<NDIM, T>(p, k, j, i, inb, W + r * PZ + x, WV, in_range);
+            flags |= load_prim<NDIM, T, vel_low<REC, LIM>()>(p, k, j, i, inb, W + r * PZ + x, WV, in_range);
         }
     }
     in_range = __syncthreads_and(in_range);
