@@ -132,8 +132,8 @@ __device__ __forceinline__ double exact_sqrt(double x) {
 //   factors 2 and fmas in place of products with a power of two are exact at these sizes;
 //   WENO5-Z: squares of differences below 2^-537 vanish, as in physics.cuh, beside the
 //   regulariser 2^-119.6; the weights are at least 1 and at most 2^650; the weighted sum is
-//   zero or at least 2^-904, and its quotient by the weights' sum normal: if the sum is
-//   large, the smooth substencil's own term, or, where that is zero, a large cell's, is too;
+//   zero or at least 2^-904, and its quotient by the weights' sum normal: where a weight is
+//   large, its own term of the sum, or, where that is zero, a large cell's, is too;
 //   kinetic energies, momentum fluxes and wave-speed terms of velocities this small are
 //   formed by the same operations as in physics.cuh, or vanish beside p >= 2^-120.
 // The face states a reconstruction makes of them are tested again before the Riemann solver
@@ -141,8 +141,9 @@ __device__ __forceinline__ double exact_sqrt(double x) {
 // the integer pipe for each value, none of the FP64 pipe.
 // Velocities decay to nothing ahead of a front in a uniform medium, so their bound is as low
 // as this allows: KH 2048^2 with the velocities across the flow times 1e-200, WENO5-Z, 2.64
-// -> 1.40 ms per step against a bound of 2^-250. Denormal ones stay out: Sedov 256^3 has
-// them in 5 to 7 % of its tiles from step 20 on and takes 2.4 % longer there than before.
+// -> 1.38 ms per step against a bound of 2^-250. Denormal ones stay out: Sedov 256^3 has
+// them in 5 to 7 % of its tiles from step 20 on and takes 7.42 ms per step at step 10, 7.56 at
+// 20, 7.59 at 40 and 7.65 at 80 (10.15 throughout with IEEE divisions).
 constexpr unsigned kVelLow = 0x0df00000u;         // upper word of 2^-800
 constexpr unsigned kVelLowVanLeer = 0x25b00000u;  // 2^-420
 template <int REC, int LIM>

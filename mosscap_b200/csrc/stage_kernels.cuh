@@ -479,11 +479,12 @@ __host__ __device__ constexpr int recon_group() {
 // neighbouring cells along the axis in shared memory, `vstride` between
 // variables. The axis is a runtime value so that both directions run the
 // same instructions.
-template <int NDIM, int REC, int LIM, int RS, class T, int G = recon_group<NDIM, REC>()>
+template <int NDIM, int REC, int LIM, int RS, class T>
 __device__ __forceinline__ void face_sweep(const T* centre, int stride, int vstride, int ntracer, T gamma, T gfac,
                                            int axis, T* d, T* d_tr) {
     constexpr int nh = 2 + NDIM;
     constexpr int S = stencil_half<REC>();
+    constexpr int G = recon_group<NDIM, REC>();
     T wl[nh], wr[nh];
     if constexpr (G < nh) {
         // a rolled loop over groups of G variables (a smaller instruction
@@ -553,25 +554,6 @@ __device__ __forceinline__ void face_sweep(const T* centre, int stride, int vstr
         const T ft = (f[0] >= T(0)) ? f[0] * tleft : f[0] * tl;
         const T fn = __shfl_down_sync(0xffffffffu, ft, 1);
         d_tr[t] = ft - fn;
-    }
-}
-
-// face_sweep on double in a call of its own: d into out[0..nh), the tracers'
-// d_tr after it. The FP64 sweep's form for values out of range. G: variables per
-// iteration of its loop; what it needs shows in its callers' registers (see
-// ztile3d_kernel).
-template <int NDIM, int REC, int LIM, int RS, int G>
-__device__ __noinline__ void face_sweep_any(const double* centre, int stride, int vstride, int ntracer, double gamma,
-                                            double gfac, int axis, double* out) {
-    constexpr int nh = 2 + NDIM;
-    double d[nh], d_tr[kMaxVars];
-    face_sweep<NDIM, REC, LIM, RS, double, G>(centre, stride, vstride, ntracer, gamma, gfac, axis, d, d_tr);
-#pragma unroll
-    for (int v = 0; v < nh; ++v) {
-        out[v] = d[v];
-    }
-    for (int t = 0; t < ntracer; ++t) {
-        out[nh + t] = d_tr[t];
     }
 }
 
@@ -657,12 +639,15 @@ __device__ __forceinline__ bool fast_face_sweep(const double* centre, int stride
 // The sweep of one line by one warp: face_sweep's result. in_range
 // (warp-uniform): every value the line's stencils read is in range; cells: the
 // number of cells from lane 1 on whose divergence is wanted; a line
-// that is not, or whose face states are not, takes face_sweep's own code.
-template <int NDIM, int REC, int LIM, int RS, class T, int GA = recon_group<NDIM, REC>()>
+// that is not, or whose face states are not, takes face_sweep's own code. (Inlined: as a
+// function of its own it made every line slower, KH 2048^2 step MUSCL 0.831 -> 0.809 ms, van
+// Leer 0.870 -> 0.839, PPM 1.002 -> 0.985, WENO5-Z 1.356 -> 1.339, Sedov 256^3 7.63 -> 7.42, and
+// those out of range by 3 to 6 %.) A whole state out of range (KH 2048^2 times 1e-45) takes
+// 1.03, 1.13, 1.11 and 1.86 ms, with IEEE arithmetic alone 1.07, 1.16, 1.08 and 1.82.
+template <int NDIM, int REC, int LIM, int RS, class T>
 __device__ __forceinline__ void sweep_line(const StageParams& p, bool in_range, int cells, const T* centre,
                                            int stride, int vstride, T gamma, T gfac, int axis, T* d, T* d_tr) {
     if constexpr (sizeof(T) == 8) {
-        constexpr int nh = 2 + NDIM;
         bool redo = true;
         if (in_range) {
             redo = !fast_face_sweep<NDIM, REC, LIM, RS>(centre, stride, vstride, p.ntracer, p.gamma, p.gas, axis, d,
@@ -671,14 +656,28 @@ __device__ __forceinline__ void sweep_line(const StageParams& p, bool in_range, 
         // only the faces of the line's cells count: lanes 1 .. cells + 1
         const int lane = threadIdx.x & 31;
         if (__any_sync(0xffffffffu, redo && lane >= 1 && lane <= cells + 1)) {
-            double out[kMaxVars];
-            face_sweep_any<NDIM, REC, LIM, RS, GA>(centre, stride, vstride, p.ntracer, gamma, gfac, axis, out);
+            if constexpr (NDIM == 2 && REC == kWeno5z) {
+                // through arrays of its own: KH 2048^2 step 1.339 ms, 1.367 without (MUSCL
+                // and PPM are up to 1 % faster without)
+                double da[2 + NDIM], dt[kMaxVars];
+                face_sweep<NDIM, REC, LIM, RS, double>(centre, stride, vstride, p.ntracer, gamma, gfac, axis, da, dt);
+                double out[kMaxVars];
 #pragma unroll
-            for (int v = 0; v < nh; ++v) {
-                d[v] = out[v];
-            }
-            for (int t = 0; t < p.ntracer; ++t) {
-                d_tr[t] = out[nh + t];
+                for (int v = 0; v < 2 + NDIM; ++v) {
+                    out[v] = da[v];
+                }
+                for (int t = 0; t < p.ntracer; ++t) {
+                    out[2 + NDIM + t] = dt[t];
+                }
+#pragma unroll
+                for (int v = 0; v < 2 + NDIM; ++v) {
+                    d[v] = out[v];
+                }
+                for (int t = 0; t < p.ntracer; ++t) {
+                    d_tr[t] = out[2 + NDIM + t];
+                }
+            } else {
+                face_sweep<NDIM, REC, LIM, RS, double>(centre, stride, vstride, p.ntracer, gamma, gfac, axis, d, d_tr);
             }
         }
     } else {
@@ -1352,14 +1351,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks2d)
     const int c = lane - 1;  // this lane's cell along the column
 
     // phase 2: z sweeps, one warp per column; the divergence replaces the
-    // column's primitives once every lane has read its stencil. The out-of-range
-    // form one variable per iteration: Sedov 256^3 FP64 z pass 1.18 -> 1.14 ms (the
-    // plane pass is slower with it, 1.33 -> 1.35)
+    // column's primitives once every lane has read its stencil
 #pragma unroll 1
     for (int col = warp; col < vw; col += kWarps) {
         T* centre = W + (c + H) * PZ + col;
         T d[nh], d_tr[kMaxVars];
-        sweep_line<NDIM, REC, LIM, RS, T, 1>(p, in_range, vh, centre, PZ, WV, gamma, gfac, 2, d, d_tr);
+        sweep_line<NDIM, REC, LIM, RS, T>(p, in_range, vh, centre, PZ, WV, gamma, gfac, 2, d, d_tr);
         __syncwarp();
         if (lane >= 1 && lane <= TZ) {
 #pragma unroll
