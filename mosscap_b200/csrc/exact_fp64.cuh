@@ -160,8 +160,9 @@ __device__ __forceinline__ bool in_range_magnitude(double x) {
 // x, a quotient with numerator n.
 template <unsigned LOW>
 __device__ __forceinline__ bool in_range_any(double x, double n) {
-    return in_range_magnitude<LOW>(x) ||
-           (((unsigned)__double2hiint(n) & 0x7fffffffu) | (unsigned)__double2loint(n)) == 0u;
+    // (no branch: the loads of the next values do not wait)
+    return in_range_magnitude<LOW>(x) |
+           ((((unsigned)__double2hiint(n) & 0x7fffffffu) | (unsigned)__double2loint(n)) == 0u);
 }
 // Four upper words of positive values at once.
 __device__ __forceinline__ bool in_range_pos4(double a, double b, double c, double d) {

@@ -125,7 +125,7 @@ __device__ __forceinline__ void run_segment(const StageParams& p, bool last, int
                 if (t < p.ntracer) {
                     const Real s = Real(q[nh + t] * inv_rho);
                     W[(nh + t) * WN + it] = s;
-                    in_range = in_range && (sizeof(Real) == 4 || in_range_any<vel_low<REC, LIM>()>(s, s));
+                    in_range &= sizeof(Real) == 4 || in_range_any<vel_low<REC, LIM>()>(s, s);
                 }
             }
         }

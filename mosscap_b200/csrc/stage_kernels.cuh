@@ -399,7 +399,7 @@ __device__ __forceinline__ unsigned store_prim(const StageParams& p, int k, int 
             const T s = T(qt * inv_rho);
             w_smem[(nh + t) * var_stride] = s;
             if constexpr (sizeof(T) == 8) {
-                in_range = in_range && in_range_any<LOW>(s, s);
+                in_range &= in_range_any<LOW>(s, s);
             }
         }
     }
