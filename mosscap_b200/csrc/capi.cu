@@ -562,13 +562,29 @@ mc_status step_host_pipelined(mc_ctx* c, double* Qh, double* Q, const mc_clock* 
 
 // Whether the device-driven loop takes its steps in the one-launch form of small
 // 1D problems (run1d_impl.cuh): no work between the stages but the stage kernel's own.
-// us per step, separate launches -> one launch (FP64): MUSCL + HLLC, rk2, 64 cells 20.5 ->
-// 6.9, 1024 17.4 -> 7.3, 3840 17.8 -> 9.2, 7680 21.5 -> 15.4; WENO5-Z + HLLC, ssprk3, 1024
-// 29.7 -> 11.7, 3840 27.6 -> 16.7, 7680 30.1 -> 30.0; beyond 256 segments (7680 cells) eight
-// SMs take longer than the launches.
+// us per step, separate launches -> one launch (FP64): MUSCL + HLLC, rk2, 64 cells 18.9 ->
+// 7.2, 960 20.6 -> 7.3, 3840 20.5 -> 9.5, 7680 20.6 -> 15.5; PPM + HLL, ssprk3, 23.6 -> 9.4 at 960,
+// 27.7 -> 13.4, 26.2 -> 23.6; WENO5-Z + HLLC, ssprk3, 29.7 -> 10.3, 29.6 -> 16.3, 29.7 -> 28.9;
+// FP32 is ahead everywhere (WENO5-Z, 7680, no tracers 25.7 -> 19.5, five 34.8 -> 30.5). Beyond
+// 256 segments (7680 cells) eight SMs take longer than the launches, and with tracers in
+// FP64 sooner: WENO5-Z, two tracers, 4800 31.8 -> 30.3, 5760 32.2 -> 32.3, 7680 32.8 -> 37.3; five
+// 3840 40.0 -> 26.5, 4800 38.4 -> 39.6, 7680 37.9 -> 51.4; PPM, two 7680 31.8 -> 30.3, five 5760
+// 36.3 -> 33.8, 6720 35.9 -> 37.3, 7680 35.8 -> 40.4.
+int run1d_segments(const mc_ctx* c) {
+    const int nt = c->grid.num_tracers;
+    if (c->scheme.precision == MC_PRECISION_FP64 && nt >= 2) {
+        if (c->scheme.reconstruction == MC_RECON_WENO5Z) {
+            return 224 - 14 * nt;
+        }
+        if (c->scheme.reconstruction == MC_RECON_PPM && nt >= 5) {
+            return 200;
+        }
+    }
+    return mc::kRun1dMaxSegments;
+}
 bool runs_whole_steps(const mc_ctx* c) {
     return c->grid.num_dim == 1 && c->eos_type == mc::kEosIdeal && !c->user_bc && !c->slab && !c->cfl_hook &&
-           !c->profiling && (c->nx + mc::kTile - 1) / mc::kTile <= mc::kRun1dMaxSegments;
+           !c->profiling && (c->nx + mc::kTile - 1) / mc::kTile <= run1d_segments(c);
 }
 
 mc_status enqueue_run1d(mc_ctx* c, double* Q, int64_t steps, double* dt_log, cudaStream_t s) {
