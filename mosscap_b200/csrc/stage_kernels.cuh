@@ -843,9 +843,10 @@ __device__ __forceinline__ void tile2d(const StageParams& p, int bx, int by, int
     }
     bool in_range = p.gas.ok != 0;
     if constexpr (TMA) {
-        // the box of WX x WY cells around the tile (x start even: the host
-        // only takes this path when ng - H is even), all hydro variables;
-        // cells outside the array arrive as zeros and are replaced below
+        // the box of SX x (th + 2 H) cells around the tile, all hydro variables. It starts
+        // at an even x: at ng - H, or, where that is odd (MUSCL with ng = 3), xo = 1 column
+        // before; with the other halos the host takes this path for even ng - H only. Cells
+        // outside the array arrive as zeros and are replaced below
         if (threadIdx.x == 0) {
             mbar_init(mbar, 1);
         }
