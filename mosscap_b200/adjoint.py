@@ -51,15 +51,17 @@ def pad_periodic(q: torch.Tensor, ng: int) -> torch.Tensor:
     return q.unsqueeze(1).contiguous()
 
 
-def torch_memory() -> capi.McAllocator:
-    """Device memory from torch's caching allocator, for the current stream. A
+def torch_memory(failures: list) -> capi.McAllocator:
+    """Device memory from torch's caching allocator, for the current stream; an
+    exception of it is appended to ``failures`` (it cannot pass through C). A
     differentiable pass makes and drops its adjoint; with cudaMalloc and cudaFree
     these took 6 of the 20 ms of a 20-step pass on 512^2. Here the memory goes
     back to torch, which has it for other tensors and frees it when it runs out."""
     def alloc(user, n):
         try:
             return torch.cuda.caching_allocator_alloc(n)
-        except torch.OutOfMemoryError:
+        except Exception as e:  # noqa: BLE001
+            failures.append(e)
             return None
 
     def free(user, p):
@@ -76,12 +78,18 @@ class _Runner:
         self.problem = problem
         self.grid = grid_of(problem)
         self.scheme = _scheme(problem, gamma)
-        self.memory = torch_memory()
+        self.failures = []
+        self.memory = torch_memory(self.failures)
         h = ctypes.c_void_p()
-        capi.check(self.lib.mc_adjoint_create_in(ctypes.byref(self.grid), ctypes.byref(self.scheme),
-                                                 int(checkpoint_every), ctypes.byref(self.memory), ctypes.byref(h)),
-                   "mc_adjoint_create_in")
+        self._check(self.lib.mc_adjoint_create_in(ctypes.byref(self.grid), ctypes.byref(self.scheme),
+                                                  int(checkpoint_every), ctypes.byref(self.memory), ctypes.byref(h)),
+                    "mc_adjoint_create_in")
         self.h = h
+
+    def _check(self, status: int, what: str) -> None:
+        if status and self.failures:
+            raise self.failures.pop()
+        capi.check(status, what)
 
     def __del__(self):
         if getattr(self, "h", None):
@@ -95,8 +103,8 @@ class _Runner:
         clk = capi.McClock()
         clk.time, clk.max_time = 0.0, 1e300
         clk.prev_output_time, clk.output_delta = 0.0, 1e300
-        capi.check(self.lib.mc_adjoint_forward(self.h, ctypes.c_void_p(qpad.data_ptr()), ctypes.byref(clk),
-                                               int(n_steps), self.stream()), "mc_adjoint_forward")
+        self._check(self.lib.mc_adjoint_forward(self.h, ctypes.c_void_p(qpad.data_ptr()), ctypes.byref(clk),
+                                                int(n_steps), self.stream()), "mc_adjoint_forward")
 
     def backward(self, lam: torch.Tensor) -> float:
         g = ctypes.c_double()

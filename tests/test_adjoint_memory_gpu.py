@@ -1,6 +1,7 @@
 """The discrete adjoint's device memory: the gradient does not depend on what it held
 before nor on work of another stream, and every block goes back to where it came from."""
 import ctypes
+import gc
 
 import pytest
 import torch
@@ -115,6 +116,33 @@ def test_memory_goes_back(gpu_lib):
     assert torch.cuda.memory_allocated() == allocated
     torch.cuda.empty_cache()
     assert free - torch.cuda.mem_get_info()[0] < 8 << 20
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("calls", [0, 3, 15])
+def test_torch_running_out_of_memory_is_its_own_error(gpu_lib, monkeypatch, calls):
+    """In mc_adjoint_create_in (0, 3) and in mc_adjoint_forward (15); the next pass works."""
+    from mosscap_b200.adjoint import kh_vy
+    p = P.kelvin_helmholtz_2d(16)
+    vy = torch.tensor(kh_vy(p), device="cuda")
+    want, _ = _gradient(p, vy, 5)
+    real, left = torch.cuda.caching_allocator_alloc, [calls]
+
+    def alloc(n):
+        if left[0] == 0:
+            raise torch.OutOfMemoryError("planned")
+        left[0] -= 1
+        return real(n)
+
+    before = torch.cuda.memory_allocated()
+    with monkeypatch.context() as m:
+        m.setattr(torch.cuda, "caching_allocator_alloc", alloc)
+        with pytest.raises(torch.OutOfMemoryError, match="planned"):
+            _gradient(p, vy, 5)
+    gc.collect()
+    assert torch.cuda.memory_allocated() == before
+    got, _ = _gradient(p, vy, 5)
+    assert torch.equal(got, want)
 
 
 def test_allocator_needs_both_functions():
